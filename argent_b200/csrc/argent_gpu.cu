@@ -1215,27 +1215,27 @@ std::vector<dev::WaveDesc> plan_waves(const std::vector<dev::DevJob>& jobs, cons
     if (P == 0 || count == 0) continue;
     uint32_t depth = 0;
     for (uint32_t j : g) depth = std::max(depth, jobs[j].max_depth);
-    // A group takes the samples per pixel and wave that one of its renders
-    // would take alone in an empty wave (sn1), on fewer pixels per wave: the
-    // film then sums every pixel's samples in the same runs as the render
-    // alone, so its values are the same bit for bit.
-    const uint64_t pn1 = std::min<uint64_t>(P, cap);
-    const uint64_t sn1 = k > 1 ? std::max<uint64_t>(1, std::min<uint64_t>(count, cap / pn1)) : count;
-    uint32_t pn_max = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(P, cap / (k * (k > 1 ? sn1 : 1))));
+    // Pixels per wave: as many as leave room for WAVE_RUN samples of each
+    // (all of them when the pass has fewer), in chunks of equal size.
+    const uint64_t run = std::min<uint64_t>(count, WAVE_RUN);
+    const uint64_t pn_cap = std::max<uint64_t>(1, std::min<uint64_t>(P, cap / (k * run)));
+    const uint64_t chunks = (P + pn_cap - 1) / pn_cap;
+    const uint32_t pn_max = (uint32_t)((P + chunks - 1) / chunks);
     for (uint32_t p0 = 0; p0 < P; p0 += pn_max) {
       uint32_t pn = std::min(pn_max, P - p0);
       uint32_t s0 = 0;
       while (s0 < count) {
-        uint64_t room = cap - cur.num_slots;
-        uint64_t want = k > 1 ? std::min<uint64_t>(count - s0, sn1) : 1;
+        // The samples that fit in the wave's free slots: the rest of the
+        // pass, or a multiple of FILM_RUN, so that the film's groups of
+        // samples are the same however the pass is cut.
+        auto fits = [&]() -> uint64_t {
+          uint64_t n = std::min<uint64_t>(count - s0, (cap - cur.num_slots) / (k * pn));
+          return n < count - s0 ? n / FILM_RUN * FILM_RUN : n;
+        };
         bool clash = false;
         for (uint32_t j : g) clash = clash || clashes(j, p0, pn);
-        if (room < k * pn * want || cur.num_segments + k > ARGENT_MAX_SEGMENTS || clash) {
-          flush();
-          room = cap;
-        }
-        uint32_t sn = (uint32_t)std::min<uint64_t>(count - s0, room / (k * pn));
-        if (k > 1) sn = (uint32_t)std::min<uint64_t>(sn, sn1);
+        if (fits() == 0 || cur.num_segments + k > ARGENT_MAX_SEGMENTS || clash) flush();
+        uint32_t sn = (uint32_t)fits();
         const uint32_t lead = cur.num_slots;
         for (uint64_t m = 0; m < k; ++m) {
           dev::DevSegment& sg = cur.seg[cur.num_segments++];
@@ -1311,10 +1311,12 @@ static int run_jobs(ArgentCtx* ctx, const std::vector<dev::DevJob>& jobs, const 
   int rc = ensure_tables(ctx);
   if (rc != ARGENT_OK) return rc;
   // Waves of up to wave_paths slots; a call with fewer path-samples than
-  // that plans one wave of its own size (at least 2^16 slots).
+  // that plans one wave of its own size (at least 2^16 slots).  A wave holds
+  // one film run of one pixel for a whole sharing group at the least.
   uint64_t total = 0;
   for (size_t j = 0; j < jobs.size(); ++j) total += (uint64_t)jobs[j].w * jobs[j].h * counts[j];
-  uint32_t cap = (uint32_t)std::min<uint64_t>(ctx->limits.wave_paths, std::max<uint64_t>(total, 1u << 16));
+  uint32_t cap = (uint32_t)std::max<uint64_t>(
+      16 * FILM_RUN, std::min<uint64_t>(ctx->limits.wave_paths, std::max<uint64_t>(total, 1u << 16)));
   std::vector<uint32_t> depths;
   const std::vector<std::vector<uint32_t>> groups = plan_groups(ctx->share_rays, jobs, counts, job_scenes);
   std::vector<dev::WaveDesc> waves = plan_waves(jobs, counts, groups, cap, &depths);

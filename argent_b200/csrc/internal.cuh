@@ -92,17 +92,30 @@ struct DevJob {
 };
 
 // A contiguous run of path slots in a wave: pixels [p0, p0+pn) of job
-// `job`, samples first+s0 .. first+s0+sn-1; slot = slot_begin + k*pn + p.
+// `job`, samples first+s0 .. first+s0+sn-1, a pixel's samples side by side:
+// slot = slot_begin + p*sn + k.  A warp's camera rays then run through one
+// pixel (or a few neighbours), so they visit the same nodes and triangles,
+// meet the same materials and send their next rays from the same spot.
+// Against a pass over the pixels per sample (slot = p + k*pn), the signet
+// still's closest-hit kernel went from 171 to 159 ms per frame and its shadow
+// rays from 86 to 79 ms (alone on the device), the gems' from 43.4 to 38.4
+// and 18.2 to 16.0 ms.
 // With ray sharing, the segments of jobs that trace the same rays (same
 // piece, camera, seed and samples; other materials) follow each other with
 // the same pixels and samples, and `lead` is the first such segment's
-// slot_begin (the slot of the same pixel-sample there is lead + k*pn + p);
+// slot_begin (the slot of the same pixel-sample there is lead + p*sn + k);
 // ~0u when the segment leads or shares nothing.
 struct DevSegment {
   uint32_t slot_begin, job, p0, pn, s0, sn, lead;
 };
 
 #define ARGENT_MAX_SEGMENTS 64
+// Samples of a pixel that the film adds as one group (k_film); every
+// segment starts at a multiple of it.
+#define FILM_RUN 8
+// Samples per pixel that the planner puts side by side in a wave when the
+// pass has as many: a warp of one pixel.
+#define WAVE_RUN 32
 struct WaveDesc {
   uint32_t num_segments;
   uint32_t num_slots;
