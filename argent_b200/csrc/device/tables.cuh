@@ -17,8 +17,9 @@ __device__ float d_energy_table[32 * 32];
 // CIE 1931 2-degree colour matching functions, 1 nm, 360..=830 (cie.rs:38-49).
 __device__ float d_cmf[471 * 3];
 // Traversal instrumentation (off unless the host enables it): closest-hit
-// rays, nodes, triangles; any-hit rays, nodes, triangles.
-__device__ int d_trav_counting;
+// rays, nodes, triangles; any-hit rays, nodes, triangles.  The switch is in
+// constant memory: every node visit tests it.
+__constant__ int d_trav_counting;
 __device__ unsigned long long d_trav_counts[6];
 // Rays by node visits (bins 0, 1, 2-3, 4-7, 8-15, 16-63, 64-255, 256+),
 // closest-hit then any-hit, and the largest visit count of each kind.

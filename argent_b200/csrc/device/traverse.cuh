@@ -200,49 +200,77 @@ __device__ __forceinline__ uint32_t child_ref(const NodeView& n, int c) {
   return ARGENT_LEAF_BIT | (cnt1 << 27) | (n.tri_base + off);
 }
 
-// Byte c of the packed plane words (w0: children 0-3, w1: 4-7) as an exact
-// float, without an integer-to-float conversion (those issue on the narrow
-// XU pipe): the byte is placed in the mantissa of 2^23, and 2^23 is
-// subtracted exactly.
+// Byte c of the packed plane words (w0: children 0-3, w1: 4-7) as the exact
+// float 2^15 + byte, in one byte permute (integer-to-float conversions issue
+// on the narrow XU pipe): the byte lands on the mantissa bits of weight 1.
+// The slab test's biases absorb the 2^15 (AxisQ).
+#define ARGENT_PLANE_BIAS 32768.0f
 __device__ __forceinline__ float qf(uint32_t w0, uint32_t w1, int c) {
-  return __fadd_rn(__uint_as_float(__byte_perm(c < 4 ? w0 : w1, 0x4B000000u, 0x7440u | (uint32_t)(c & 3))),
-                   -8388608.0f);
+  return __uint_as_float(__byte_perm(c < 4 ? w0 : w1, 0x47000000u, 0x7604u | ((uint32_t)(c & 3) << 4)));
 }
 
 // A ray prepared for the node-space slab test: the inverse direction with
-// magnitudes capped at 2^64 (a zero component gives +-2^64, so no 0 * inf
-// arises), and per axis whether the ray runs toward -axis.
+// magnitudes capped (a zero component gives +-cap, so no 0 * inf arises),
+// and per axis whether the ray runs toward -axis.
 struct RayQ {
   V3 o;
   float ix, iy, iz;
   bool nx, ny, nz;
 };
 
-__device__ __forceinline__ float capped_inv(float d) {
-  const float cap = 18446744073709551616.0f;  // 2^64
-  return fminf(fmaxf(__fdiv_rn(1.0f, d), -cap), cap);
+// The inverses come from the hardware's reciprocal estimate (1 ulp): the slab
+// interval's slack covers its error many times over, and hits do not depend
+// on the boxes beyond their being entered.
+__device__ __forceinline__ float capped_inv(float d, float cap) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  return fminf(fmaxf(r, -cap), cap);
 }
 
-__device__ __forceinline__ RayQ make_rayq(V3 o, V3 d) {
+// `root` is the word of the root node with its exponent bytes: pieces whose
+// boxes are so large that scale * cap * 2^15 could overflow (scale >= 2^33)
+// take a smaller cap.
+__device__ __forceinline__ RayQ make_rayq(V3 o, V3 d, uint32_t root) {
+  const bool big = (root & ((root << 1) | (root << 2)) & 0x00808080u) != 0;
+  const float cap = big ? 281474976710656.0f : 18446744073709551616.0f;  // 2^48, 2^64
   RayQ r;
   r.o = o;
-  r.ix = capped_inv(d.x);
-  r.iy = capped_inv(d.y);
-  r.iz = capped_inv(d.z);
+  r.ix = capped_inv(d.x, cap);
+  r.iy = capped_inv(d.y, cap);
+  r.iz = capped_inv(d.z, cap);
   r.nx = signbit(r.ix);
   r.ny = signbit(r.iy);
   r.nz = signbit(r.iz);
   return r;
 }
 
+// Three-operand minimum and maximum (one instruction on sm_100; a NaN operand
+// is dropped, as fminf and fmaxf drop it).
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
 // One axis of a node seen from a ray.  A plane q of the axis is at
 // t = (origin + q * scale - o) * inv = q * a + b, with a = scale * inv
-// (exact: scale is a power of two) and b = (origin - o) * inv.  Computed as
-// fma(q, a, b), t differs from the exact value by at most about
-// 3 * 2^-24 * (|origin - o| + 255 * scale) * |inv|; the slack e is 2^-18
-// times that magnitude (64 units of rounding), and is subtracted from the
-// near plane's bias and added to the far plane's.  The near plane is the
-// low one unless the ray runs toward -axis.
+// (exact: scale is a power of two) and b = (origin - o) * inv.  It is
+// computed from the decoded v = 2^15 + q as fma(v, a, b'), b' = b - 2^15 a.
+// Against the exact value that is off by at most about
+// 2^-21 * |origin - o| * |inv| + 2^-9 * |a| (the roundings of b and b', the
+// inverse's ulp, the final rounding); the slack e = 2^-18 * |origin - o| *
+// |inv| + 2^-7 * |a| is over four times that, and is subtracted from the
+// near plane's bias and added to the far plane's (1/128 of a quantisation
+// step).  The near plane is the low one unless the ray runs toward -axis.
+// The traversals are bound by issue, the narrow integer pipe first, so the
+// decode is one permute, the bounds take three-operand min and max, and
+// children are counted from the sorted keys: the signet still's closest hit
+// went from 159.7 to 154.0 ms per frame, its shadow rays from 79.3 to 76.4.
 struct AxisQ {
   float a, bn, bf;
   uint32_t n0, n1, f0, f1;
@@ -253,10 +281,10 @@ __device__ __forceinline__ AxisQ axis_q(float origin, float scale, float o, floa
   AxisQ q;
   float dd = __fsub_rn(origin, o);
   float b = __fmul_rn(dd, inv);
-  float e = __fmul_rn(__fmul_rn(__fadd_rn(fabsf(dd), __fmul_rn(256.0f, scale)), fabsf(inv)), 3.814697265625e-06f);
+  float e = __fmul_rn(__fmaf_rn(fabsf(dd), 3.814697265625e-06f, __fmul_rn(scale, 0.0078125f)), fabsf(inv));
   q.a = __fmul_rn(scale, inv);
-  q.bn = __fsub_rn(b, e);
-  q.bf = __fadd_rn(b, e);
+  q.bn = __fmaf_rn(-ARGENT_PLANE_BIAS, q.a, __fsub_rn(b, e));
+  q.bf = __fmaf_rn(-ARGENT_PLANE_BIAS, q.a, __fadd_rn(b, e));
   q.n0 = neg ? hi0 : lo0;
   q.n1 = neg ? hi1 : lo1;
   q.f0 = neg ? lo0 : hi0;
@@ -270,9 +298,8 @@ struct NodeQ {
 
 // The whole box of a node, planes 0 and 255 on every axis (it holds every
 // child box), with the slack of axis_q.  Reads only the node's first 16
-// bytes.  A ray that misses the root's box misses the piece.
-__device__ __forceinline__ bool node_box_hit(const uint4* nodes, uint32_t idx, const RayQ& r, float t_max) {
-  uint4 w0 = ld_node16(nodes + 5 * (size_t)idx);
+// bytes (w0).  A ray that misses the root's box misses the piece.
+__device__ __forceinline__ bool node_box_hit(uint4 w0, const RayQ& r, float t_max) {
   float o[3] = {__uint_as_float(w0.x), __uint_as_float(w0.y), __uint_as_float(w0.z)};
   float ro[3] = {r.o.x, r.o.y, r.o.z};
   float iv[3] = {r.ix, r.iy, r.iz};
@@ -307,8 +334,8 @@ __device__ __forceinline__ bool child_q(const NodeQ& q, int c, float t_max, floa
   float tfx = __fmaf_rn(qf(q.x.f0, q.x.f1, c), q.x.a, q.x.bf);
   float tfy = __fmaf_rn(qf(q.y.f0, q.y.f1, c), q.y.a, q.y.bf);
   float tfz = __fmaf_rn(qf(q.z.f0, q.z.f1, c), q.z.a, q.z.bf);
-  float tmin = fmaxf(fmaxf(tnx, tny), fmaxf(tnz, 0.0f));
-  float tmax = fminf(fminf(tfx, tfy), fminf(tfz, t_max));
+  float tmin = fmaxf(max3(tnx, tny, tnz), 0.0f);
+  float tmax = fminf(min3(tfx, tfy, tfz), t_max);
   *tmin_out = tmin;
   return tmin <= tmax;
 }
@@ -386,22 +413,13 @@ __device__ __forceinline__ void sort8(uint32_t k[8]) {
 }
 #undef ARGENT_CX
 
-// Children's push order: 1 = all entered children sorted by entry distance
-// (the nearest popped first), 0 = the nearest entered at once and the rest
-// pushed in slot order.  Hits do not depend on it (see below).  Measured on
-// B200 with eight lanes: sorted 1.752 G path-samples/s on the signet still
-// and 1.17 G on the gems, nearest-first 1.737 G and 1.144 G (it visits a
-// few more nodes, and needs a few more registers), so sorting stays.
-#ifndef ARGENT_SORTED_PUSH
-#define ARGENT_SORTED_PUSH 1
-#endif
-
 // Closest hit with t in (1e-7, t_max).  Ties at equal t go to the lower
 // original triangle index.
 //
 // Order of visits: of the children a node's slab test keeps, the nearest
-// by entry distance is entered at once; the others are pushed with their
-// entry distances (ARGENT_SORTED_PUSH: far-to-near).  The key is the entry
+// by entry distance is entered at once; the others are pushed far to near
+// with their entry distances (entering the nearest and pushing the rest in
+// slot order visits a few more nodes and ran slower).  The key is the entry
 // distance with its 3 low mantissa bits replaced by the child slot; the
 // truncated distance is what the stack keeps for pruning, which can only
 // keep more nodes than the exact value.
@@ -438,8 +456,9 @@ __device__ __forceinline__ bool closest_begin(const DevPiece& pc, ClosestTrav& s
   s.n_nodes = 0;
   s.n_tris = 0;
   if (pc.num_tris == 0) return false;
-  s.rq = make_rayq(o, d);
-  if (!node_box_hit(pc.nodes, 0u, s.rq, t_max)) return false;
+  const uint4 root = ld_node16(pc.nodes);
+  s.rq = make_rayq(o, d, root.w);
+  if (!node_box_hit(root, s.rq, t_max)) return false;
   s.have = true;
   return true;
 }
@@ -492,49 +511,32 @@ __device__ __forceinline__ bool closest_visit(const DevPiece& pc, ClosestTrav& s
   ++s.n_nodes;
   NodeQ nq = node_ray(n, s.rq);
   uint32_t k[8];
-  int nh = 0;
-  uint32_t hm = 0;
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
     float tc;
     bool h = child_q(nq, c, s.best.t, &tc) && ((n.present >> c) & 1u);
     k[c] = h ? ((__float_as_uint(tc) & ~7u) | (uint32_t)c) : 0xFFFFFFFFu;
-    nh += h ? 1 : 0;
-    hm |= h ? (1u << c) : 0u;
   }
-  if (d_trav_counting) atomicAdd(&d_trav_child_hits[nh], 1ull);
-  if (nh == 0) return s.sp > 0;
-  if (s.sp + nh - 1 > ARGENT_STACK_SIZE) {
+  if (d_trav_counting) {
+    int nh = 0;
+    for (int c = 0; c < 8; ++c) nh += k[c] != 0xFFFFFFFFu ? 1 : 0;
+    atomicAdd(&d_trav_child_hits[nh], 1ull);
+  }
+  sort8(k);
+  if (k[0] == 0xFFFFFFFFu) return s.sp > 0;
+  // Pieces are refused at upload unless 7 entries per level of their tree
+  // fit, so a visit that could overflow the stack is an error whatever its
+  // children.
+  if (s.sp + 7 > ARGENT_STACK_SIZE) {
     atomicOr(status, ARGENT_STATUS_STACK_OVERFLOW);
     s.sp = 0;
     return false;
   }
-#if ARGENT_SORTED_PUSH
-  sort8(k);
 #pragma unroll
   for (int j = 7; j >= 1; --j) {
-    if (j < nh) stack.push(s.sp, make_uint2(child_ref(n, (int)(k[j] & 7u)), k[j] & ~7u));
+    if (k[j] != 0xFFFFFFFFu) stack.push(s.sp, make_uint2(child_ref(n, (int)(k[j] & 7u)), k[j] & ~7u));
   }
   s.ref = child_ref(n, (int)(k[0] & 7u));
-#else
-  // Descend into the nearest child; push the others (nh - 1: none in three
-  // visits of four, and at most one in more than nine of ten) in slot order
-  // with their entry distances, so popping still prunes them against the
-  // running best.  The loop runs as many times as the lane has children to
-  // push, where the sort costs 19 compare-exchanges and eight guarded
-  // pushes on every visit.
-  uint32_t kmin = min(min(min(k[0], k[1]), min(k[2], k[3])), min(min(k[4], k[5]), min(k[6], k[7])));
-  uint32_t near = kmin & 7u;
-  uint32_t rest = hm & ~(1u << near);
-  while (rest) {
-    int c = __ffs(rest) - 1;
-    rest &= rest - 1u;
-    uint32_t kc = c == 0 ? k[0] : c == 1 ? k[1] : c == 2 ? k[2] : c == 3 ? k[3]
-                : c == 4 ? k[4] : c == 5 ? k[5] : c == 6 ? k[6] : k[7];
-    stack.push(s.sp, make_uint2(child_ref(n, c), kc & ~7u));
-  }
-  s.ref = child_ref(n, (int)near);
-#endif
   s.have = true;
   return true;
 }
@@ -577,7 +579,8 @@ struct AnyTrav {
 // (up to t_max) misses its box, so nothing of the piece can occlude it.
 __device__ __forceinline__ bool piece_may_occlude(const DevPiece& pc, V3 o, V3 d, float t_max) {
   if (pc.num_tris == 0) return false;
-  return node_box_hit(pc.nodes, 0u, make_rayq(o, d), t_max);
+  const uint4 root = ld_node16(pc.nodes);
+  return node_box_hit(root, make_rayq(o, d, root.w), t_max);
 }
 
 // Returns ARGENT_ANY_RUNNING, or ARGENT_ANY_CLEAR when the ray misses the
@@ -592,8 +595,9 @@ __device__ __forceinline__ int any_begin(const DevPiece& pc, AnyTrav& s, ST& sta
   s.n_nodes = 0;
   s.n_tris = 0;
   if (pc.num_tris == 0) return ARGENT_ANY_CLEAR;
-  s.rq = make_rayq(o, d);
-  if (!node_box_hit(pc.nodes, 0u, s.rq, t_max)) return ARGENT_ANY_CLEAR;
+  const uint4 root = ld_node16(pc.nodes);
+  s.rq = make_rayq(o, d, root.w);
+  if (!node_box_hit(root, s.rq, t_max)) return ARGENT_ANY_CLEAR;
   stack.push(s.sp, 0u);
   return ARGENT_ANY_RUNNING;
 }

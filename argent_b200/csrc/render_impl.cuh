@@ -94,7 +94,10 @@ __device__ __forceinline__ Spec panel_le(const DevPanel& p, V3 x, V3 dir, const 
 // light.rs:142-148
 __device__ __forceinline__ bool floor_intersect(const DevScene* sc, V3 o, V3 d, float t_max, float* t_out) {
   if (fabsf(d.y) < 1e-9f) return false;
-  float t = (sc->floor_y - o.y) / d.y;
+  float num = sc->floor_y - o.y;
+  // As in panel_intersect: t <= 0 without the division.
+  if (num == 0.0f || (signbit(num) != signbit(d.y))) return false;
+  float t = num / d.y;
   if (t > 1e-5f && t < t_max) {
     *t_out = t;
     return true;
