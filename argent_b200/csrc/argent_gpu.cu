@@ -83,6 +83,46 @@ __global__ void k_trace_any(DevPiece pc, const ArgentRay* __restrict__ rays, uin
   }
 }
 
+// The same for calls too small to fill the device with a thread per ray:
+// eight lanes per ray (coop_trace), all rays at once.
+__global__ void __launch_bounds__(128) k_trace_closest_few(DevPiece pc, const ArgentRay* __restrict__ rays, uint32_t n,
+                                                           ArgentHit* hits, uint32_t* status) {
+  const uint32_t j = coop_entry(n, gridDim.x * (blockDim.x >> 5));
+  const bool active = j != ~0u;
+  if (__ballot_sync(0xffffffffu, active) == 0) return;
+  uint2 arr[ARGENT_STACK_SIZE];
+  LocalStack<uint2> stack{arr};
+  float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
+  if (active) {
+    const float4* rp = reinterpret_cast<const float4*>(rays + j);
+    a = __ldg(rp);
+    b = __ldg(rp + 1);
+  }
+  TraceHit h = coop_trace<false>(pc, stack, active, V3{a.x, a.y, a.z}, V3{b.x, b.y, b.z}, a.w, status);
+  if (active && (threadIdx.x & (ARGENT_COOP_GROUP - 1)) == 0) {
+    const bool miss = h.prim == ARGENT_NO_HIT_U;
+    reinterpret_cast<float4*>(hits)[j] =
+        make_float4(miss ? 0.0f : h.t, miss ? 0.0f : h.u, miss ? 0.0f : h.v, __uint_as_float(h.prim));
+  }
+}
+
+__global__ void __launch_bounds__(128) k_trace_any_few(DevPiece pc, const ArgentRay* __restrict__ rays, uint32_t n,
+                                                       uint8_t* occ, uint32_t* status) {
+  const uint32_t j = coop_entry(n, gridDim.x * (blockDim.x >> 5));
+  const bool active = j != ~0u;
+  if (__ballot_sync(0xffffffffu, active) == 0) return;
+  uint2 arr[ARGENT_STACK_SIZE];
+  LocalStack<uint2> stack{arr};
+  float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
+  if (active) {
+    const float4* rp = reinterpret_cast<const float4*>(rays + j);
+    a = __ldg(rp);
+    b = __ldg(rp + 1);
+  }
+  TraceHit h = coop_trace<true>(pc, stack, active, V3{a.x, a.y, a.z}, V3{b.x, b.y, b.z}, a.w, status);
+  if (active && (threadIdx.x & (ARGENT_COOP_GROUP - 1)) == 0) occ[j] = h.prim != ARGENT_NO_HIT_U ? 1 : 0;
+}
+
 // Rewrites every triangle record of a piece for a triangle test: (v0, e1,
 // e2) with e = v - v0 rounded as the host builder rounds it (argent's
 // Moller-Trumbore), or the three original vertices (v0, v1, v2) marked
@@ -176,6 +216,15 @@ int grid_for(const ArgentCtx* ctx, const void* kernel, int block, uint64_t n) {
   uint64_t full = (n + block - 1) / block;
   uint64_t g = std::min<uint64_t>(full, (uint64_t)ctx->num_sms * per_sm);
   return (int)std::max<uint64_t>(g, 1);
+}
+
+// Blocks of 128 threads for the eight-lanes-per-ray form of a trace of `n`
+// rays (every ray at once, one per warp while warps are free), or 0 when the
+// call has enough rays to fill the device with a thread each.
+static int few_rays_grid(const ArgentCtx* ctx, uint64_t n) {
+  const uint64_t blocks = (uint64_t)ctx->num_sms * ARGENT_TRAV_BLOCKS;
+  if (n > blocks * 4 * ARGENT_COOP_RAYS) return 0;
+  return (int)std::min<uint64_t>(blocks, (n + 3) / 4);
 }
 
 // ------------------------------------------------------------------ kernel timing
@@ -635,17 +684,23 @@ uint64_t argent_piece_device_bytes(const ArgentPiece* p) { return p ? p->bytes :
 
 // ------------------------------------------------------------------ traversal entry points
 
+static void launch_trace_closest(ArgentCtx* ctx, ArgentPiece* piece, const ArgentRay* d_rays, uint64_t n,
+                                 ArgentHit* d_hits) {
+  const int few = few_rays_grid(ctx, n);
+  ProfScope ps(ctx, KC_TRACE);
+  if (few)
+    k_trace_closest_few<<<few, 128, 0, ctx->stream>>>(piece->dev, d_rays, (uint32_t)n, d_hits, ctx->d_status);
+  else
+    k_trace_closest<<<grid_for(ctx, (const void*)k_trace_closest, 128, n), 128, 0, ctx->stream>>>(
+        piece->dev, d_rays, n, d_hits, ctx->d_status);
+}
+
 int argent_trace_closest_device(ArgentCtx* ctx, ArgentPiece* piece, const ArgentRay* d_rays, uint64_t n,
                                 ArgentHit* d_hits) {
   if (!ctx || !piece) return set_error(ctx, ARGENT_E_INVALID, "NULL argument");
   if (n == 0) return ARGENT_OK;
   ARGENT_CK(ctx, cudaSetDevice(ctx->device));
-  int block = 128;
-  int grid = grid_for(ctx, (const void*)k_trace_closest, block, n);
-  {
-    ProfScope ps(ctx, KC_TRACE);
-    k_trace_closest<<<grid, block, 0, ctx->stream>>>(piece->dev, d_rays, n, d_hits, ctx->d_status);
-  }
+  launch_trace_closest(ctx, piece, d_rays, n, d_hits);
   ctx->launches++;
   ARGENT_CK(ctx, cudaGetLastError());
   return ARGENT_OK;
@@ -656,11 +711,14 @@ int argent_trace_anyhit_device(ArgentCtx* ctx, ArgentPiece* piece, const ArgentR
   if (!ctx || !piece) return set_error(ctx, ARGENT_E_INVALID, "NULL argument");
   if (n == 0) return ARGENT_OK;
   ARGENT_CK(ctx, cudaSetDevice(ctx->device));
-  int block = 128;
-  int grid = grid_for(ctx, (const void*)k_trace_any, block, n);
+  const int few = few_rays_grid(ctx, n);
   {
     ProfScope ps(ctx, KC_TRACE);
-    k_trace_any<<<grid, block, 0, ctx->stream>>>(piece->dev, d_rays, n, d_occ, ctx->d_status);
+    if (few)
+      k_trace_any_few<<<few, 128, 0, ctx->stream>>>(piece->dev, d_rays, (uint32_t)n, d_occ, ctx->d_status);
+    else
+      k_trace_any<<<grid_for(ctx, (const void*)k_trace_any, 128, n), 128, 0, ctx->stream>>>(piece->dev, d_rays, n,
+                                                                                          d_occ, ctx->d_status);
   }
   ctx->launches++;
   ARGENT_CK(ctx, cudaGetLastError());
@@ -2655,12 +2713,7 @@ extern "C" int argent_trace_closest_noalloc(ArgentCtx* ctx, ArgentPiece* piece, 
   // Every hit the call returns is written by the kernel, so nothing in the
   // array has to start at zero; rays are overwritten by this copy.
   ARGENT_CK(ctx, cudaMemcpyAsync(d_rays, rays, n * sizeof(ArgentRay), cudaMemcpyHostToDevice, ctx->stream));
-  int block = 128;
-  int grid = grid_for(ctx, (const void*)k_trace_closest, block, n);
-  {
-    ProfScope ps(ctx, KC_TRACE);
-    k_trace_closest<<<grid, block, 0, ctx->stream>>>(piece->dev, d_rays, n, d_hits, ctx->d_status);
-  }
+  launch_trace_closest(ctx, piece, d_rays, n, d_hits);
   ctx->launches++;
   ARGENT_CK(ctx, cudaGetLastError());
   ARGENT_CK(ctx, cudaMemcpyAsync(hits, d_hits, n * sizeof(ArgentHit), cudaMemcpyDeviceToHost, ctx->stream));

@@ -340,40 +340,14 @@ __device__ __forceinline__ bool child_q(const NodeQ& q, int c, float t_max, floa
   return tmin <= tmax;
 }
 
-// Traversal stacks.  LocalStack keeps a thread's whole stack in its local
-// memory.  ShortStack keeps the top S entries in shared memory (a ring per
-// thread: entry k in row k % S of the thread's column, so the 32 threads of
-// a warp touch 32 consecutive words and no bank twice) and moves older
-// entries to a local-memory spill array only while the stack is deeper than
-// S: a push that wraps onto an occupied row first writes that row's entry to
-// spill[sp - S], and a pop that uncovers a spilled entry moves it back into
-// the freed row.  The order of entries is the same either way, so
-// traversals, pruning and results do not depend on the stack kind.
+// A thread's traversal stack, in its local memory (it hits in L1; rings of 8
+// or 16 entries in shared memory ran slower, as their 8-16 KB per block cost
+// the other lanes' kernels L1 and co-residency).
 template <typename E>
 struct LocalStack {
   E* a;
   __device__ __forceinline__ void push(int& sp, E e) { a[sp++] = e; }
   __device__ __forceinline__ E pop(int& sp) { return a[--sp]; }
-};
-
-template <typename E, int S, int STRIDE>
-struct ShortStack {
-  static_assert((S & (S - 1)) == 0, "ring size must be a power of two");
-  E* sh;     // this thread's column in the block's shared ring array
-  E* spill;  // this thread's local spill array
-  __device__ __forceinline__ void push(int& sp, E e) {
-    E* row = sh + (sp & (S - 1)) * STRIDE;
-    if (sp >= S) spill[sp - S] = *row;
-    *row = e;
-    ++sp;
-  }
-  __device__ __forceinline__ E pop(int& sp) {
-    --sp;
-    E* row = sh + (sp & (S - 1)) * STRIDE;
-    E e = *row;
-    if (sp >= S) *row = spill[sp - S];
-    return e;
-  }
 };
 
 struct TraceHit {
@@ -430,8 +404,7 @@ __device__ __forceinline__ void sort8(uint32_t k[8]) {
 // The traversal is resumable: closest_begin sets it up and each
 // closest_step visits one node or one leaf, so a kernel can interleave the
 // steps of rays that start at different times (persistent lanes that take a
-// new ray as soon as theirs finishes).  The stack (LocalStack or
-// ShortStack) lives with the caller.
+// new ray as soon as theirs finishes).  The stack lives with the caller.
 struct ClosestTrav {
   V3 o, d;
   RayQ rq;
@@ -668,6 +641,245 @@ __device__ __noinline__ bool trace_any(const DevPiece& pc, V3 o, V3 d, float t_m
   while (r == ARGENT_ANY_RUNNING) r = any_step(pc, s, stack, status);
   count_visits(3, s.n_nodes, s.n_tris);
   return r == ARGENT_ANY_HIT;
+}
+
+// ---------------------------------------------------------------- few rays
+// Traversal by groups of eight lanes, for queues too short to fill the
+// device: a lane per child of a node and per triangle of a leaf, so a ray's
+// chain of steps is several times shorter in time (a lone lane takes the
+// eight slab tests, the sort and the leaf's triangles one after the other).
+// All lanes of a warp call together; the lanes of a group pass the same ray.
+// The hits are those of trace_closest and trace_any: the closest hit is the
+// minimum of (t, triangle index) whatever the order of visits, and the boxes
+// are tested by the same arithmetic.
+//
+// Rays are dealt to warps one by one first (coop_rays_per_warp), so with
+// fewer rays than warps the groups of a warp do not wait for each other.
+// Bound by the latency of a step (a node's or leaf's loads from L2, then one
+// child or triangle per lane), with the device mostly idle either way.  The
+// preview (512 x 512, 4 spp, 500k triangles) spent 1.61 ms in its 12 closest
+// hit launches and 1.05 ms in its shadow rays, 1.21 and 0.75 ms with it; the
+// render went from 3.47 to 2.83 ms.  The form is taken up to 4 rays per
+// resident warp, where every ray still runs at once; above that a thread per
+// ray holds eight times as many rays in flight per warp.
+#define ARGENT_COOP_GROUP 8
+#define ARGENT_COOP_RAYS (32 / ARGENT_COOP_GROUP)  // rays a warp holds at most
+
+// Rays per warp when `warps` warps take `count` rays in one go (count <=
+// ARGENT_COOP_RAYS * warps).
+__host__ __device__ inline uint32_t coop_rays_per_warp(uint32_t count, uint32_t warps) {
+  return (count + warps - 1) / warps;
+}
+
+// A traversal that a group shares: every lane of the group holds the same
+// values, but the stack, which is the group's first lane's.
+struct CoopTrav {
+  V3 o, d;
+  RayQ rq;
+  float t_max;
+  TraceHit best;
+  uint32_t ref;  // the node or leaf to visit next, if `have`
+  int sp;
+  bool run, have;
+  uint32_t n_nodes, n_tris;
+};
+
+__device__ __forceinline__ void coop_begin(const DevPiece& pc, CoopTrav& s, bool active, V3 o, V3 d, float t_max) {
+  s.o = o;
+  s.d = d;
+  s.t_max = t_max;
+  s.best = TraceHit{t_max, 0.0f, 0.0f, ARGENT_NO_HIT_U};
+  s.ref = 0;
+  s.sp = 0;
+  s.n_nodes = s.n_tris = 0;
+  s.run = false;
+  if (active && pc.num_tris != 0) {
+    const uint4 root = ld_node16(pc.nodes);
+    s.rq = make_rayq(o, d, root.w);
+    s.run = node_box_hit(root, s.rq, t_max);
+  }
+  s.have = s.run;
+}
+
+// Runs the groups' traversals to their ends.  ANY stops a ray at its first
+// hit and leaves 0 in best.prim (ARGENT_NO_HIT_U: clear).
+template <bool ANY, class ST>
+__device__ __forceinline__ void coop_run(const DevPiece& pc, CoopTrav& s, ST& stack, uint32_t* status) {
+  const unsigned full = 0xffffffffu, gmask = (1u << ARGENT_COOP_GROUP) - 1u;
+  const unsigned c = threadIdx.x & (ARGENT_COOP_GROUP - 1);    // this lane's child, triangle
+  const unsigned g0 = threadIdx.x & (32 - ARGENT_COOP_GROUP);  // the group's first lane
+  for (;;) {
+    // Groups without a node or leaf at hand take theirs from the stack.
+    if (__ballot_sync(full, s.run && !s.have)) {
+      if (s.run && !s.have && c == 0) {
+        while (s.sp > 0) {
+          uint2 e = stack.pop(s.sp);
+          if (__uint_as_float(e.y) <= s.best.t) {
+            s.ref = e.x;
+            s.have = true;
+            break;
+          }
+        }
+      }
+      s.sp = __shfl_sync(full, s.sp, (int)g0);
+      s.ref = __shfl_sync(full, s.ref, (int)g0);
+      s.have = __shfl_sync(full, s.have ? 1 : 0, (int)g0) != 0;
+      s.run = s.run && s.have;
+    }
+    if (__ballot_sync(full, s.run) == 0) break;
+    const uint32_t ref = s.ref;
+    const bool leaf = (ref & ARGENT_LEAF_BIT) != 0;
+    s.have = false;
+    if (__ballot_sync(full, s.run && !leaf)) {
+      uint32_t key = 0xFFFFFFFFu, cref = 0;
+      if (s.run && !leaf) {
+        NodeView n = load_node(pc.nodes, ref);
+        ++s.n_nodes;
+        NodeQ nq = node_ray(n, s.rq);
+        const bool hi = c >= 4;
+        // This lane's child as byte c & 3 of the first plane words.
+        nq.x.n0 = hi ? nq.x.n1 : nq.x.n0;
+        nq.y.n0 = hi ? nq.y.n1 : nq.y.n0;
+        nq.z.n0 = hi ? nq.z.n1 : nq.z.n0;
+        nq.x.f0 = hi ? nq.x.f1 : nq.x.f0;
+        nq.y.f0 = hi ? nq.y.f1 : nq.y.f0;
+        nq.z.f0 = hi ? nq.z.f1 : nq.z.f0;
+        float tc;
+        if (child_q(nq, (int)(c & 3), s.best.t, &tc) && ((n.present >> c) & 1u)) {
+          key = (__float_as_uint(tc) & ~7u) | c;
+          cref = child_ref(n, (int)c);
+        }
+      }
+      // Rank of this lane's child among the group's entered children.
+      uint32_t rank = 0;
+#pragma unroll
+      for (int i = 1; i < ARGENT_COOP_GROUP; ++i)
+        rank += __shfl_xor_sync(full, key, i) < key ? 1u : 0u;
+      const bool in = key != 0xFFFFFFFFu;
+      // Far to near onto the stack; the nearest (rank 0) is entered next.
+      const int nh = __popc((__ballot_sync(full, in) >> g0) & gmask);
+      if (s.run && s.sp + nh > ARGENT_STACK_SIZE) {  // refused at upload (see closest_visit)
+        if (c == 0) atomicOr(status, ARGENT_STATUS_STACK_OVERFLOW);
+        s.sp = 0;
+      }
+      for (int r = 1; __ballot_sync(full, r < nh); ++r) {
+        // Entry r from the far end: rank nh - r.
+        const unsigned gm = (__ballot_sync(full, in && (int)rank == nh - r) >> g0) & gmask;
+        const int src = (int)g0 + (gm ? __ffs(gm) - 1 : 0);
+        const uint32_t rr = __shfl_sync(full, cref, src), kk = __shfl_sync(full, key, src);
+        if (r < nh) {
+          if (c == 0)
+            stack.push(s.sp, make_uint2(rr, kk & ~7u));
+          else
+            ++s.sp;
+        }
+      }
+      const unsigned gn = (__ballot_sync(full, in && rank == 0) >> g0) & gmask;
+      const uint32_t next = __shfl_sync(full, cref, (int)g0 + (gn ? __ffs(gn) - 1 : 0));
+      if (nh > 0) {
+        s.ref = next;
+        s.have = true;
+      }
+    }
+    if (__ballot_sync(full, s.run && leaf)) {
+      const uint32_t cnt = s.run && leaf ? ((ref >> 27) & 15u) + 1u : 0u;
+      s.n_tris += cnt;
+      for (uint32_t i0 = 0; __ballot_sync(full, i0 < cnt); i0 += ARGENT_COOP_GROUP) {
+        float t = 0.0f, u = 0.0f, v = 0.0f;
+        uint32_t prim = 0;
+        // (t, triangle index) as one ordered word; t > 1e-7, so its bits
+        // order as its values.
+        unsigned long long key = ~0ull;
+        if (i0 + c < cnt && mt_hit(pc.tris + 3 * (size_t)((ref & 0x07FFFFFFu) + i0 + c), s.o, s.d, s.t_max, &t, &u,
+                                   &v, &prim))
+          key = ((unsigned long long)__float_as_uint(t) << 32) | prim;
+        const unsigned hm = (__ballot_sync(full, key != ~0ull) >> g0) & gmask;
+        if (ANY) {
+          if (hm) {
+            s.best.prim = 0;
+            s.run = false;
+          }
+          continue;
+        }
+        unsigned long long mn = key;
+#pragma unroll
+        for (int i = 1; i < ARGENT_COOP_GROUP; i <<= 1) {
+          const unsigned long long x = __shfl_xor_sync(full, mn, i);
+          mn = x < mn ? x : mn;
+        }
+        const unsigned wm = (__ballot_sync(full, key == mn) >> g0) & gmask;
+        const int src = (int)g0 + __ffs(wm) - 1;
+        u = __shfl_sync(full, u, src);
+        v = __shfl_sync(full, v, src);
+        if (hm) {
+          t = __uint_as_float((uint32_t)(mn >> 32));
+          prim = (uint32_t)mn;
+          if (t < s.best.t || (t == s.best.t && prim < s.best.prim)) s.best = TraceHit{t, u, v, prim};
+        }
+      }
+    }
+  }
+}
+
+// Hands the warp's last running any-hit rays (at most ARGENT_COOP_RAYS, the
+// lanes of `mask`) to its groups: group g takes the g-th of them, with the
+// state `st` and the stack `own` (references) its lane has reached; the
+// groups go on with `stack`.
+__device__ __forceinline__ CoopTrav coop_take(unsigned mask, const CoopTrav& st, const uint32_t* own,
+                                              LocalStack<uint2>& stack) {
+  const unsigned full = 0xffffffffu;
+  const unsigned lane = threadIdx.x & 31u;
+  unsigned m = mask;
+  for (unsigned i = 0; i < lane / ARGENT_COOP_GROUP; ++i) m &= m - 1u;
+  const bool active = m != 0;
+  const int src = active ? __ffs(m) - 1 : (int)lane;
+  auto f = [&](float x) { return __shfl_sync(full, x, src); };
+  auto u = [&](uint32_t x) { return __shfl_sync(full, x, src); };
+  CoopTrav t;
+  t.o = V3{f(st.o.x), f(st.o.y), f(st.o.z)};
+  t.d = V3{f(st.d.x), f(st.d.y), f(st.d.z)};
+  t.rq.o = t.o;
+  t.rq.ix = f(st.rq.ix);
+  t.rq.iy = f(st.rq.iy);
+  t.rq.iz = f(st.rq.iz);
+  t.rq.nx = signbit(t.rq.ix);
+  t.rq.ny = signbit(t.rq.iy);
+  t.rq.nz = signbit(t.rq.iz);
+  t.t_max = f(st.t_max);
+  t.best = TraceHit{t.t_max, 0.0f, 0.0f, ARGENT_NO_HIT_U};
+  t.ref = u(st.ref);
+  t.sp = (int)u((uint32_t)st.sp);
+  t.have = u(st.have ? 1u : 0u) != 0;
+  if (!active) {  // a lane that never had a ray holds no state
+    t.sp = 0;
+    t.have = false;
+  }
+  t.n_nodes = u(st.n_nodes);
+  t.n_tris = u(st.n_tris);
+  t.run = active;
+  for (int i = 0; __ballot_sync(full, active && i < t.sp); ++i) {
+    const uint32_t e = u(own[i]);
+    if (active && i < t.sp && (lane & (ARGENT_COOP_GROUP - 1)) == 0) stack.a[i] = make_uint2(e, 0u);
+  }
+  return t;
+}
+
+// The lane whose group holds the result of this lane's ray (a lane of
+// `mask`).
+__device__ __forceinline__ int coop_lane_of(unsigned mask) {
+  const unsigned lane = threadIdx.x & 31u;
+  return (__popc(mask & ((1u << lane) - 1u)) * ARGENT_COOP_GROUP) & 31;
+}
+
+template <bool ANY, class ST>
+__device__ __forceinline__ TraceHit coop_trace(const DevPiece& pc, ST& stack, bool active, V3 o, V3 d, float t_max,
+                                               uint32_t* status) {
+  CoopTrav s;
+  s.rq = RayQ{};
+  coop_begin(pc, s, active, o, d, t_max);
+  coop_run<ANY>(pc, s, stack, status);
+  if (active && (threadIdx.x & (ARGENT_COOP_GROUP - 1)) == 0) count_visits(ANY ? 3 : 0, s.n_nodes, s.n_tris);
+  return s.best;
 }
 
 }  // namespace dev

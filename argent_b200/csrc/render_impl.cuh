@@ -465,39 +465,101 @@ __device__ __forceinline__ uint32_t lane_refill(bool idle, bool* first, bool* mo
 // kernel of its hit's material class.  Persistent lanes step their BVH
 // traversals one node or leaf at a time and take a new path as soon as
 // theirs is done.
-// Rows of the traversal kernels' shared-memory stack rings (ShortStack);
-// 0 keeps the whole stack in local memory.  The kernels run 128 threads per
-// block.  Measured on B200 (signet still, eight lanes): local stacks 1.756 G
-// path-samples/s, rings of 8 rows 1.727 G, of 16 rows 1.722 G -- the rings'
-// shared memory (8-16 KB per block) costs the other lanes' kernels L1 and
-// co-residency more than the stack traffic it saves (the local stack hits
-// in L1), so the default is 0.
-#ifndef ARGENT_SHORT_STACK
-#define ARGENT_SHORT_STACK 0
-#endif
-#ifndef ARGENT_SHORT_STACK_ANY
-#define ARGENT_SHORT_STACK_ANY 0
-#endif
-#if ARGENT_SHORT_STACK > 0
-#define ARGENT_CLOSEST_STACK(name)                                             \
-  __shared__ uint2 name##_ring[ARGENT_SHORT_STACK * 128];                      \
-  uint2 name##_spill[ARGENT_STACK_SIZE];                                       \
-  ShortStack<uint2, ARGENT_SHORT_STACK, 128> name{name##_ring + threadIdx.x, name##_spill}
-#else
-#define ARGENT_CLOSEST_STACK(name)   \
-  uint2 name##_arr[ARGENT_STACK_SIZE]; \
-  LocalStack<uint2> name { name##_arr }
-#endif
-#if ARGENT_SHORT_STACK_ANY > 0
-#define ARGENT_ANY_STACK(name)                                                     \
-  __shared__ uint32_t name##_ring[ARGENT_SHORT_STACK_ANY * 128];                   \
-  uint32_t name##_spill[ARGENT_STACK_SIZE];                                        \
-  ShortStack<uint32_t, ARGENT_SHORT_STACK_ANY, 128> name{name##_ring + threadIdx.x, name##_spill}
-#else
-#define ARGENT_ANY_STACK(name)          \
-  uint32_t name##_arr[ARGENT_STACK_SIZE]; \
-  LocalStack<uint32_t> name { name##_arr }
-#endif
+// Eight lanes per ray, every ray of the queue at once (coop_trace): a queue
+// of up to 4 rays per resident warp leaves the device mostly idle, and its
+// time is that of its slowest ray.
+// The entry this lane's group takes, or ~0u.
+__device__ __forceinline__ uint32_t coop_entry(uint32_t count, uint32_t warps) {
+  const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const uint32_t per = coop_rays_per_warp(count, warps), g = (threadIdx.x & 31u) / ARGENT_COOP_GROUP;
+  const uint32_t j = warp * per + g;
+  return g < per && j < count ? j : ~0u;
+}
+
+// The lane whose ray this lane's group takes in coop_take(mask), or -1.
+__device__ __forceinline__ int coop_owner(unsigned mask) {
+  for (unsigned i = 0; i < (threadIdx.x & 31u) / ARGENT_COOP_GROUP; ++i) mask &= mask - 1u;
+  return mask ? __ffs(mask) - 1 : -1;
+}
+// The piece that path `slot` of lane `owner` traces (waves of several scenes).
+__device__ __forceinline__ DevPiece coop_piece(const WaveArgs& a, uint32_t slot, int owner) {
+  const uint32_t s = __shfl_sync(0xffffffffu, slot, owner < 0 ? 0 : owner);
+  DevPiece pc{};
+  if (owner >= 0) pc = a.jobs[a.meta[s].w >> 16].scene->piece;
+  return pc;
+}
+
+template <bool U>
+__device__ __forceinline__ void intersect_few(const WaveArgs& a, int depth, uint32_t count, uint32_t warps,
+                                              const uint32_t* qin, LocalStack<uint2>& stack) {
+  const uint32_t j = coop_entry(count, warps);
+  const bool active = j != ~0u;
+  if (__ballot_sync(0xffffffffu, active) == 0) return;
+  const unsigned c = threadIdx.x & (ARGENT_COOP_GROUP - 1);
+  const DevScene* sc = U ? a.uscene : nullptr;
+  uint32_t slot = 0;
+  V3 o{0.0f, 0.0f, 0.0f}, d{0.0f, 0.0f, 1.0f};
+  if (active) {
+    slot = qin[j];
+    if (!U) sc = a.jobs[a.meta[slot].w >> 16].scene;
+    float4 of = a.o[slot], df = a.d[slot];
+    o = V3{of.x, of.y, of.z};
+    d = V3{df.x, df.y, df.z};
+  }
+  V3 oo = o, od = d;
+  if (active && (U ? a.u_has_turn : sc->has_turn)) {
+    float ts = U ? a.u_to_obj_s : sc->to_obj_s, tc = U ? a.u_to_obj_c : sc->to_obj_c;
+    oo = rot_y_sc(o, ts, tc);
+    od = rot_y_sc(d, ts, tc);
+  }
+  DevPiece pc = a.upiece;
+  if (!U && active) pc = sc->piece;
+  const TraceHit best = coop_trace<false>(pc, stack, active, oo, od, INFINITY, a.status);
+  // Panels: a lane per panel, then the nearest (the first of equals, as the
+  // one-by-one test keeps it).
+  const float t_piece = best.prim != ARGENT_NO_HIT_U ? best.t : INFINITY;
+  unsigned long long pk = ~0ull;
+  if (active) {
+    for (int p = (int)c; p < sc->num_panels; p += ARGENT_COOP_GROUP) {
+      const DevPanel& pn = sc->panels[p];
+      if (depth == 0 && !pn.camera_visible) continue;
+      float t;
+      if (panel_intersect(pn, o, d, t_piece, &t)) {
+        const unsigned long long x = ((unsigned long long)__float_as_uint(t) << 32) | (uint32_t)p;
+        pk = x < pk ? x : pk;
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 1; i < ARGENT_COOP_GROUP; i <<= 1) {
+    const unsigned long long x = __shfl_xor_sync(0xffffffffu, pk, i);
+    pk = x < pk ? x : pk;
+  }
+  int cls = -1;
+  if (active && c == 0) {
+    float t_max = t_piece;
+    float4 rec = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(HIT_MISS));
+    cls = CLS_TERMINAL;
+    if (pk != ~0ull) {
+      t_max = __uint_as_float((uint32_t)(pk >> 32));
+      rec = make_float4(t_max, 0.0f, 0.0f, __uint_as_float(HIT_PANEL | (uint32_t)pk));
+    } else if (best.prim != ARGENT_NO_HIT_U) {
+      rec = make_float4(best.t, best.u, best.v, __uint_as_float(best.prim));
+      cls = sc->mat_class[__ldg(&pc.tri_idx[best.prim].w)];
+    }
+    if (sc->floor_enabled) {
+      float t;
+      if (floor_intersect(sc, o, d, t_max, &t)) {
+        rec = make_float4(t, 0.0f, 0.0f, __uint_as_float(HIT_FLOOR));
+        cls = sc->floor_class;
+      }
+    }
+    a.hit[slot] = rec;
+  }
+#pragma unroll
+  for (int k = 0; k < NUM_CLS; ++k)
+    warp_append(cls == k, slot, a.counters + CNT_CLS(depth, k), a.qc + (size_t)k * a.cap, a.cap, a.status);
+}
 
 template <bool U>
 __global__ void __launch_bounds__(128, ARGENT_TRAV_BLOCKS) k_intersect(WaveArgs a, int depth) {
@@ -507,7 +569,13 @@ __global__ void __launch_bounds__(128, ARGENT_TRAV_BLOCKS) k_intersect(WaveArgs 
   const uint32_t count = a.counters[cq];
   uint32_t* work = a.counters + CNT_WORK(cq);
   const uint32_t* qin = a.lead ? a.qt : a.q_in;
-  ARGENT_CLOSEST_STACK(stack);
+  uint2 stack_arr[ARGENT_STACK_SIZE];
+  LocalStack<uint2> stack{stack_arr};
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  if (count <= ARGENT_COOP_RAYS * warps) {
+    intersect_few<U>(a, depth, count, warps, qin, stack);
+    return;
+  }
   ClosestTrav s;
   const DevScene* sc = U ? a.uscene : nullptr;
   uint32_t slot = 0;
@@ -1027,6 +1095,39 @@ __global__ void __launch_bounds__(128, CLS == CLS_TERMINAL      ? 1
   }
 }
 
+// Adds a clear shadow record's contribution to its path's radiance.
+__device__ __forceinline__ void add_shadow(const WaveArgs& a, uint32_t idx) {
+  uint32_t slot = __float_as_uint(__ldcs(a.sh_d + idx).w);
+  float4 c = __ldcs(a.sh_c + idx);
+  float4 l = a.L[slot];
+  a.L[slot] = make_float4(l.x + c.x, l.y + c.y, l.z + c.z, l.w + c.w);
+}
+
+// As intersect_few, for the shadow queue.
+template <bool U>
+__device__ __forceinline__ void shadow_few(const WaveArgs& a, uint32_t count, uint32_t warps,
+                                           LocalStack<uint2>& stack) {
+  const uint32_t j = coop_entry(count, warps);
+  const bool active = j != ~0u;
+  if (__ballot_sync(0xffffffffu, active) == 0) return;
+  uint32_t idx = 0;
+  float4 so = make_float4(0.0f, 0.0f, 0.0f, 0.0f), sd = so;
+  DevPiece pc = a.upiece;
+  if (active) {
+    idx = a.lead ? a.qst[j] : j;
+    so = __ldcs(a.sh_o + idx);
+    sd = __ldcs(a.sh_d + idx);
+    if (!U) pc = a.jobs[a.meta[__float_as_uint(sd.w)].w >> 16].scene->piece;
+  }
+  const TraceHit h =
+      coop_trace<true>(pc, stack, active, V3{so.x, so.y, so.z}, V3{sd.x, sd.y, sd.z}, so.w, a.status);
+  if (active && (threadIdx.x & (ARGENT_COOP_GROUP - 1)) == 0) {
+    const bool clear = h.prim == ARGENT_NO_HIT_U;
+    if (a.vis) a.vis[idx] = clear ? 1u : 0u;
+    if (clear) add_shadow(a, idx);
+  }
+}
+
 // scene.rs:123-140 (piece part): any hit of the piece for each shadow ray;
 // unoccluded rays add their contribution to L.  Persistent lanes, so a
 // lane whose ray ends early takes a new one instead of idling until the
@@ -1039,7 +1140,15 @@ __global__ void __launch_bounds__(128, ARGENT_TRAV_BLOCKS) k_shadow(WaveArgs a, 
   const uint32_t cq = a.lead ? CNT_STR(depth) : CNT_SH(depth);
   const uint32_t count = a.counters[cq];
   uint32_t* work = a.counters + CNT_WORK(cq);
-  ARGENT_ANY_STACK(stack);
+  uint2 coop_arr[ARGENT_STACK_SIZE];
+  LocalStack<uint2> coop_stack{coop_arr};
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5);
+  if (count <= ARGENT_COOP_RAYS * warps) {
+    shadow_few<U>(a, count, warps, coop_stack);
+    return;
+  }
+  uint32_t stack_arr[ARGENT_STACK_SIZE];
+  LocalStack<uint32_t> stack{stack_arr};
   AnyTrav s;
   const DevScene* sc = nullptr;
   uint32_t idx = 0;
@@ -1063,15 +1172,32 @@ __global__ void __launch_bounds__(128, ARGENT_TRAV_BLOCKS) k_shadow(WaveArgs a, 
       bool leaves = __popc(__ballot_sync(0xffffffffu, at_leaf)) >= __popc(__ballot_sync(0xffffffffu, at_node));
       if (leaves ? at_leaf : at_node) state = any_visit(U ? a.upiece : sc->piece, s, stack, a.status);
     }
+    // The queue is empty and at most four of the warp's rays still run: a
+    // long ray is finished by eight lanes instead of one.  (In k_intersect
+    // the same made the main loop spill and the signet still 3 % slower.)
+    if (!more) {
+      const unsigned tail = __ballot_sync(0xffffffffu, active && state == ARGENT_ANY_RUNNING);
+      if (tail != 0 && __popc(tail) <= ARGENT_COOP_RAYS) {
+        DevPiece pc = a.upiece;
+        if (!U) pc = coop_piece(a, active ? __float_as_uint(__ldcs(a.sh_d + idx).w) : 0u, coop_owner(tail));
+        const TraceHit none{s.t_max, 0.0f, 0.0f, ARGENT_NO_HIT_U};
+        CoopTrav own{s.o, s.d, s.rq, s.t_max, none, s.ref, s.sp, true, s.have, s.n_nodes, s.n_tris};
+        CoopTrav t = coop_take(tail, own, stack_arr, coop_stack);
+        coop_run<true>(pc, t, coop_stack, a.status);
+        const int from = coop_lane_of(tail);
+        const uint32_t prim = __shfl_sync(0xffffffffu, t.best.prim, from);
+        const uint32_t nn = __shfl_sync(0xffffffffu, t.n_nodes, from), nt = __shfl_sync(0xffffffffu, t.n_tris, from);
+        if (active && state == ARGENT_ANY_RUNNING) {
+          state = prim == ARGENT_NO_HIT_U ? ARGENT_ANY_CLEAR : ARGENT_ANY_HIT;
+          s.n_nodes = nn;
+          s.n_tris = nt;
+        }
+      }
+    }
     if (active && state != ARGENT_ANY_RUNNING) {
       count_visits(3, s.n_nodes, s.n_tris);
       if (a.vis) a.vis[idx] = state == ARGENT_ANY_CLEAR ? 1u : 0u;
-      if (state == ARGENT_ANY_CLEAR) {
-        uint32_t slot = __float_as_uint(__ldcs(a.sh_d + idx).w);
-        float4 c = __ldcs(a.sh_c + idx);
-        float4 l = a.L[slot];
-        a.L[slot] = make_float4(l.x + c.x, l.y + c.y, l.z + c.z, l.w + c.w);
-      }
+      if (state == ARGENT_ANY_CLEAR) add_shadow(a, idx);
       active = false;
     }
   }
