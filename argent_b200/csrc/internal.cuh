@@ -183,6 +183,7 @@ struct KernelProfile {
 // idle.  Lane 0 runs on the context stream.
 #define ARGENT_LANES 16
 #define ARGENT_GRAPH_CACHE 8
+#define ARGENT_SIDES 4
 
 struct ArgentCtx {
   int device = 0;
@@ -190,6 +191,11 @@ struct ArgentCtx {
   cudaStream_t lane_stream[ARGENT_LANES] = {};
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr;
   cudaEvent_t film_ev[ARGENT_LANES] = {};
+  // Each lane's side streams (a bounce's shading classes beside each other,
+  // and its shadow rays beside the next bounce's closest hits) and the events
+  // that tie them to the lane's stream.
+  cudaStream_t side_stream[ARGENT_LANES][ARGENT_SIDES] = {};
+  cudaEvent_t side_ev[ARGENT_LANES][ARGENT_SIDES + 1] = {};
   // Waves rotate over the lanes across calls: the next call starts at
   // next_lane, and, while an overlapped batch may still run, its first film
   // pass waits for the film pass of the last wave before it (on
