@@ -1945,6 +1945,10 @@ int argent_scene_upload(ArgentCtx* ctx, ArgentPiece* piece, const ArgentSceneDes
       dp.hv[a] = p.hv[a];
     }
     argent::panel_frame(p, dp.n, &dp.area, &dp.hu_l2, &dp.hv_l2);
+    dp.nd = dp.n[0] * dp.c[0] + dp.n[1] * dp.c[1] + dp.n[2] * dp.c[2];
+    float far = 0.0f;
+    for (int a = 0; a < 3; ++a) far += std::fabs(dp.c[a]) + std::fabs(dp.hu[a]) + std::fabs(dp.hv[a]);
+    dp.guard = far < 1e7f ? 3.814697265625e-06f * far : INFINITY;
     dp.feather = p.feather;
     dp.emits = p.emits ? 1 : 0;
     dp.camera_visible = p.camera_visible ? 1 : 0;

@@ -48,37 +48,42 @@ __device__ __forceinline__ uint32_t sobol_dim(uint32_t index, int d) {
   return __ldg(t + (index & 0xffu)) ^ __ldg(t + 256 + ((index >> 8) & 0xffu)) ^
          __ldg(t + 512 + ((index >> 16) & 0xffu)) ^ __ldg(t + 768 + (index >> 24));
 }
-__device__ __forceinline__ void sample_4d(uint32_t index, uint32_t set, uint32_t seed, float out[4]) {
+// The first N of the four values of padding set `set`.  Dimension 0 is the
+// van der Corput sequence, whose generator matrix reverses the index's bits:
+// the reversal cancels the scramble's own (the tables serve the others).
+template <int N>
+__device__ __forceinline__ void sample_4d(uint32_t index, uint32_t set, uint32_t seed, float* out) {
   uint32_t sseed = hash_combine(seed, hash32(set));
   uint32_t shuffled = nested_uniform_scramble(index, sseed);
 #pragma unroll
-  for (int d = 0; d < 4; ++d) {
-    uint32_t x = sobol_dim(shuffled, d);
-    x = nested_uniform_scramble(x, hash_combine(sseed, hash32((uint32_t)d + 1u)));
+  for (int d = 0; d < N; ++d) {
+    uint32_t dseed = hash_combine(sseed, hash32((uint32_t)d + 1u));
+    uint32_t x = d == 0 ? __brev(lk_permutation(shuffled, dseed))
+                        : nested_uniform_scramble(sobol_dim(shuffled, d), dseed);
     out[d] = (float)(x >> 8) * (1.0f / 16777216.0f);
   }
 }
 
+// argent's dimension stream is drawn in sets of four dimensions, as the
+// callers need them: a path's camera sample takes dimensions 0..4, bounce d
+// the eight from 8 + 8 d.  A set is Sobol or PCG as a whole (256 is a
+// multiple of four), and PCG values come in the order of the dimensions, so
+// the values are those of argent's one-by-one draws.  (argent clamps Sobol
+// values to 0.99999994; 24-bit values never exceed it.)
 struct Sampler {
-  uint32_t index, seed, dim;
+  uint32_t index, seed;
   uint64_t rng;
-  uint32_t block_set;
-  float block[4];
 
   __device__ __forceinline__ void init(uint32_t pixel_seed, uint32_t sample_index) {
     index = sample_index;
     seed = pixel_seed;
-    dim = 0;
     rng = (((uint64_t)pixel_seed << 32) | (uint64_t)sample_index) ^ 0x9e3779b97f4a7c15ull;
-    block_set = 0xffffffffu;
   }
   // Resume a path: the PCG state travels with the path between kernels.
   __device__ __forceinline__ void resume(uint32_t pixel_seed, uint32_t sample_index, uint64_t rng_state) {
     index = sample_index;
     seed = pixel_seed;
-    dim = 0;
     rng = rng_state;
-    block_set = 0xffffffffu;
   }
   __device__ __forceinline__ float next_random() {
     rng = rng * 6364136223846793005ull + 1442695040888963407ull;
@@ -87,22 +92,16 @@ struct Sampler {
     uint32_t v = __funnelshift_r((uint32_t)x, (uint32_t)x, rot);
     return (float)(v >> 8) * (1.0f / 16777216.0f);
   }
-  __device__ __forceinline__ float next() {
-    uint32_t d = dim;
-    dim += 1;
-    if (d < ARGENT_SOBOL_MAX_DIM && index < (1u << 16)) {
-      uint32_t set = d >> 2;
-      if (set != block_set) {
-        sample_4d(index, set, seed, block);
-        block_set = set;
-      }
-      uint32_t k = d & 3u;
-      float v = k == 0 ? block[0] : (k == 1 ? block[1] : (k == 2 ? block[2] : block[3]));
-      return fminf(v, 0.99999994f);
+  // The first N dimensions of set `set` (dimensions 4 set .. 4 set + N - 1).
+  template <int N>
+  __device__ __forceinline__ void draw(uint32_t set, float* out) {
+    if (set < ARGENT_SOBOL_MAX_DIM / 4u && index < (1u << 16)) {
+      sample_4d<N>(index, set, seed, out);
+    } else {
+#pragma unroll
+      for (int d = 0; d < N; ++d) out[d] = next_random();
     }
-    return next_random();
   }
-  __device__ __forceinline__ void set_dim(uint32_t d) { dim = d; }
 };
 
 // sampler.rs:103-108

@@ -20,8 +20,10 @@
 
 namespace dev {
 
-struct DevPanel {
-  float c[3], hu[3], hv[3], n[3];
+struct alignas(16) DevPanel {
+  float n[3], nd;  // unit normal and its product with the centre (one load: panel_near)
+  float guard;     // error bound of panel_near's plane distances
+  float c[3], hu[3], hv[3];
   float area, feather, hu_l2, hv_l2;
   int32_t emits, camera_visible;
   const float* emission;  // 471-entry table
