@@ -13,11 +13,13 @@ struct Bsdf {
   int kind;
   Ggx ggx;
   Spec eta, k;  // conductor eta/k; dielectric eta
-  // Conductor: F(1) per wavelength and E(wo.z), which argent recomputes on
-  // every eval (bsdf.rs:62-64); both depend only on the hit, so they are
-  // evaluated once per hit (same values).
-  Spec f0;
-  float e_wo;
+  // What depends on the hit alone, which argent recomputes on every eval,
+  // pdf and sample (bsdf.rs:62-78, 105-113, 164-182); bsdf_prepare evaluates
+  // it once per hit (same values).  Conductor: the energy compensation 1 +
+  // F(1) (1 - E) / E per wavelength.  Coated: the coat's Fresnel term of wo and
+  // the probability of its lobe.  Both: lambda of wo.
+  Spec ms;
+  float wo_f, wo_ps, wo_lam;
   float eta1;   // coated eta
   Spec base;    // coated base, diffuse albedo, opal body
   V3 n;         // opal lattice normal (local)
@@ -64,26 +66,57 @@ __device__ __forceinline__ float coated_pdf(Ggx ggx, float eta, const Spec& base
   return ps * p_spec + (1.0f - ps) * wi.z * ARGENT_FRAC_1_PI_F;
 }
 
-// coated_eval and coated_pdf of the same directions, sharing the half
-// vector and the Fresnel term of wo: the same values as the two calls.
-__device__ __forceinline__ void coated_eval_pdf(Ggx ggx, float eta, const Spec& base, V3 wo, V3 wi, Spec* f,
-                                                float* pdf) {
+// coated_eval and coated_pdf of the same directions, sharing the half vector
+// and the terms of wo that bsdf_prepare holds: the same values as the two
+// calls.
+__device__ __forceinline__ void coated_eval_pdf(const Bsdf& b, V3 wo, V3 wi, Spec* f, float* pdf) {
   if (wo.z <= 0.0f || wi.z <= 0.0f) {
     *f = spec(0.0f);
     *pdf = 0.0f;
     return;
   }
   V3 h = normalize(wo + wi);
-  float fo = fresnel_dielectric(wo.z, eta);
-  float fs = fresnel_dielectric(dot(wo, h), eta);
-  float sp = ggx_d(ggx, h) * ggx_g2(ggx, wo, wi) * fs / (4.0f * wo.z * wi.z);
-  float fi = fresnel_dielectric(wi.z, eta);
-  *f = base * ((1.0f - fo) * (1.0f - fi) * ARGENT_FRAC_1_PI_F) + spec(sp);
-  // coat_spec_prob(wo.z, eta, base) from the same Fresnel value
-  float d = average(base) * (1.0f - fo);
-  float ps = rclamp(fo / fmaxf(fo + d, 1e-6f), 0.15f, 0.95f);
-  float p_spec = ggx_d_visible(ggx, wo, h) / (4.0f * fmaxf(dot(wo, h), 1e-8f));
-  *pdf = ps * p_spec + (1.0f - ps) * wi.z * ARGENT_FRAC_1_PI_F;
+  float fs = fresnel_dielectric(dot(wo, h), b.eta1);
+  float d = ggx_d(b.ggx, h);
+  float sp = d * (1.0f / (1.0f + b.wo_lam + ggx_lambda(b.ggx, wi))) * fs / (4.0f * wo.z * wi.z);
+  float fi = fresnel_dielectric(wi.z, b.eta1);
+  *f = b.base * ((1.0f - b.wo_f) * (1.0f - fi) * ARGENT_FRAC_1_PI_F) + spec(sp);
+  float p_spec = ggx_d_visible_from(b.wo_lam, d, wo, h) / (4.0f * fmaxf(dot(wo, h), 1e-8f));
+  *pdf = b.wo_ps * p_spec + (1.0f - b.wo_ps) * wi.z * ARGENT_FRAC_1_PI_F;
+}
+
+// The microfacet parts of a light sample's BSDF value and pdf, alpha^2
+// D-numerator included: *spec = D G2 / (4 wo.z wi.z) (the Fresnel factor left
+// to the caller) and *pdf = the visible-normal density of the half vector over
+// 4 wo.h.  With so = wo.z sqrt(1 + a^2 tan^2 wo) and si alike, G2 / (4 wo.z
+// wi.z) = 1 / (2 (wi.z so + wo.z si)) and G1(wo) / (4 wo.z) = 1 / (2 (wo.z +
+// so)), so one division serves both where the factors one by one take nine.
+// Light samples only: their values scale radiance and steer no path.  h.z and
+// the denominator of D, whose rounding a smooth surface amplifies, are
+// computed as everywhere else.
+__device__ __forceinline__ void ggx_nee(Ggx g, float wo_lam, V3 wo, V3 wi, V3 h, float* spec_out, float* pdf) {
+  const float a2 = g.alpha * g.alpha;
+  const float c2 = h.z * h.z;
+  const float k = c2 * (a2 - 1.0f) + 1.0f;
+  const float so = wo.z * (1.0f + 2.0f * wo_lam);
+  const float si = sqrtf(__fmaf_rn(a2, fmaxf(1.0f - wi.z * wi.z, 0.0f), wi.z * wi.z));
+  const float x = __fmaf_rn(wi.z, so, wo.z * si), y = wo.z + so;
+  const float q = a2 / ((2.0f * ARGENT_PI_F) * (k * k) * (x * y));
+  *spec_out = q * y;
+  *pdf = q * x;
+}
+
+// The coat's eval and pdf for a light sample (coated_eval_pdf but for
+// rounding).
+__device__ __forceinline__ void coated_nee(const Bsdf& b, V3 wo, V3 wi, Spec* f, float* pdf) {
+  V3 h = normalize(wo + wi);
+  float sp, p_spec;
+  ggx_nee(b.ggx, b.wo_lam, wo, wi, h, &sp, &p_spec);
+  const float ie2 = 1.0f / (b.eta1 * b.eta1);
+  const float fs = fresnel_dielectric_nee(dot(wo, h), b.eta1, ie2);
+  const float fi = fresnel_dielectric_nee(wi.z, b.eta1, ie2);
+  *f = b.base * ((1.0f - b.wo_f) * (1.0f - fi) * ARGENT_FRAC_1_PI_F) + spec(sp * fs);
+  *pdf = b.wo_ps * p_spec + (1.0f - b.wo_ps) * wi.z * ARGENT_FRAC_1_PI_F;
 }
 
 // bsdf.rs:219-254
@@ -128,13 +161,11 @@ __device__ Spec bsdf_eval(const Bsdf& b, V3 wo, V3 wi) {
       if (wo.z <= 0.0f || wi.z <= 0.0f || is_smooth(b.ggx)) return spec(0.0f);
       V3 h = normalize(wo + wi);
       Spec f = fresnel_conductor(dot(wo, h), b.eta, b.k);
-      float base = ggx_d(b.ggx, h) * ggx_g2(b.ggx, wo, wi) / (4.0f * wo.z * wi.z);
-      float e = b.e_wo;
-      return f * base * (spec(1.0f) + b.f0 * ((1.0f - e) / e));
+      float base = ggx_d(b.ggx, h) * (1.0f / (1.0f + b.wo_lam + ggx_lambda(b.ggx, wi))) / (4.0f * wo.z * wi.z);
+      return f * base * b.ms;
     }
     case B_COATED:
-      if constexpr (!KM_HAS(KM, B_COATED)) return spec(0.0f);
-      return coated_eval(b.ggx, b.eta1, b.base, wo, wi);
+      return spec(0.0f);  // coated_eval_pdf
     case B_DIFFUSE:
       if constexpr (!KM_HAS(KM, B_DIFFUSE)) return spec(0.0f);
       if (wo.z <= 0.0f || wi.z <= 0.0f) return spec(0.0f);
@@ -155,15 +186,6 @@ __device__ Spec bsdf_eval(const Bsdf& b, V3 wo, V3 wi) {
 template <unsigned KM = KM_ALL>
 __device__ float bsdf_pdf(const Bsdf& b, V3 wo, V3 wi) {
   switch (b.kind) {
-    case B_CONDUCTOR: {
-      if constexpr (!KM_HAS(KM, B_CONDUCTOR)) return 0.0f;
-      if (wo.z <= 0.0f || wi.z <= 0.0f || is_smooth(b.ggx)) return 0.0f;
-      V3 h = normalize(wo + wi);
-      return ggx_d_visible(b.ggx, wo, h) / (4.0f * fmaxf(dot(wo, h), 1e-8f));
-    }
-    case B_COATED:
-      if constexpr (!KM_HAS(KM, B_COATED)) return 0.0f;
-      return coated_pdf(b.ggx, b.eta1, b.base, wo, wi);
     case B_DIFFUSE:
       if constexpr (!KM_HAS(KM, B_DIFFUSE)) return 0.0f;
       if (wo.z <= 0.0f || wi.z <= 0.0f) return 0.0f;
@@ -179,40 +201,55 @@ __device__ float bsdf_pdf(const Bsdf& b, V3 wo, V3 wi) {
   }
 }
 
-// bsdf_eval and bsdf_pdf of the same directions; conductor and coated lobes
-// share their half vector (and the coat its Fresnel term of wo).
+// Fills the terms of `b` that depend on wo alone (local frame).
 template <unsigned KM = KM_ALL>
-__device__ __forceinline__ void bsdf_eval_pdf(const Bsdf& b, V3 wo, V3 wi, Spec* f, float* pdf) {
-  if (KM_HAS(KM, B_COATED) && b.kind == B_COATED) {
-    coated_eval_pdf(b.ggx, b.eta1, b.base, wo, wi, f, pdf);
-    return;
+__device__ __forceinline__ void bsdf_prepare(Bsdf& b, V3 wo) {
+  if (KM_HAS(KM, B_COATED) && b.kind == B_COATED && wo.z > 0.0f) {
+    b.wo_f = fresnel_dielectric(wo.z, b.eta1);
+    // coat_spec_prob(wo.z, eta, base) from the same Fresnel value
+    float d = average(b.base) * (1.0f - b.wo_f);
+    b.wo_ps = rclamp(b.wo_f / fmaxf(b.wo_f + d, 1e-6f), 0.15f, 0.95f);
+    b.wo_lam = ggx_lambda(b.ggx, wo);
   }
-  if (KM_HAS(KM, B_CONDUCTOR) && b.kind == B_CONDUCTOR) {
-    if (wo.z <= 0.0f || wi.z <= 0.0f || is_smooth(b.ggx)) {
-      *f = spec(0.0f);
-      *pdf = 0.0f;
-      return;
-    }
-    V3 h = normalize(wo + wi);
-    Spec fr = fresnel_conductor(dot(wo, h), b.eta, b.k);
-    float base = ggx_d(b.ggx, h) * ggx_g2(b.ggx, wo, wi) / (4.0f * wo.z * wi.z);
-    float e = b.e_wo;
-    *f = fr * base * (spec(1.0f) + b.f0 * ((1.0f - e) / e));
-    *pdf = ggx_d_visible(b.ggx, wo, h) / (4.0f * fmaxf(dot(wo, h), 1e-8f));
-    return;
+  if (KM_HAS(KM, B_CONDUCTOR) && b.kind == B_CONDUCTOR && !is_smooth(b.ggx) && wo.z > 0.0f) {
+    Spec f0 = fresnel_conductor(1.0f, b.eta, b.k);
+    float e = ggx_e(b.ggx, wo.z);
+    b.ms = spec(1.0f) + f0 * ((1.0f - e) / e);
+    b.wo_lam = ggx_lambda(b.ggx, wo);
   }
-  *f = bsdf_eval<KM>(b, wo, wi);
-  *pdf = bsdf_pdf<KM>(b, wo, wi);
 }
 
-// Coated lobe sampling (bsdf.rs:164-182).
-__device__ __forceinline__ bool coated_sample(Ggx ggx, float eta, const Spec& base, V3 wo, float u0, float u1,
-                                              float u2, BsdfSample* out) {
+// BSDF value and pdf of a light sample's direction.
+template <unsigned KM = KM_ALL>
+__device__ __forceinline__ void bsdf_nee(const Bsdf& b, V3 wo, V3 wi, Spec* f, float* pdf) {
+  *f = spec(0.0f);
+  *pdf = 0.0f;
+  if (wo.z <= 0.0f || wi.z <= 0.0f) return;
+  if (KM_HAS(KM, B_COATED) && b.kind == B_COATED) {
+    coated_nee(b, wo, wi, f, pdf);
+  } else if (KM_HAS(KM, B_CONDUCTOR) && b.kind == B_CONDUCTOR) {
+    if (is_smooth(b.ggx)) return;
+    V3 h = normalize(wo + wi);
+    float base;
+    ggx_nee(b.ggx, b.wo_lam, wo, wi, h, &base, pdf);
+    const float c = dot(wo, h);
+    Spec fr;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) fr.v[i] = fresnel_conductor_nee(c, b.eta.v[i], b.k.v[i]);
+    *f = fr * base * b.ms;
+  } else {
+    *f = bsdf_eval<KM>(b, wo, wi);
+    *pdf = bsdf_pdf<KM>(b, wo, wi);
+  }
+}
+
+// Coated lobe sampling (bsdf.rs:164-182).  `b` holds the terms of wo
+// (bsdf_prepare).
+__device__ __forceinline__ bool coated_sample(const Bsdf& b, V3 wo, float u0, float u1, float u2, BsdfSample* out) {
   if (wo.z <= 0.0f) return false;
-  float ps = coat_spec_prob(wo.z, eta, base);
   V3 wi;
-  if (u0 < ps) {
-    V3 h = ggx_sample_h(ggx, wo, u1, u2);
+  if (u0 < b.wo_ps) {
+    V3 h = ggx_sample_h(b.ggx, wo, u1, u2);
     wi = reflect(wo, h);
   } else {
     wi = cosine_hemisphere(u1, u2);
@@ -220,7 +257,7 @@ __device__ __forceinline__ bool coated_sample(Ggx ggx, float eta, const Spec& ba
   if (wi.z <= 0.0f) return false;
   float p;
   Spec f;
-  coated_eval_pdf(ggx, eta, base, wo, wi, &f, &p);
+  coated_eval_pdf(b, wo, wi, &f, &p);
   if (p <= 0.0f) return false;
   out->wi = wi;
   out->f = f;
@@ -249,13 +286,13 @@ __device__ bool bsdf_sample(const Bsdf& b, V3 wo, float u0, float u1, float u2, 
       V3 wi = reflect(wo, h);
       if (wi.z <= 0.0f) return false;
       out->wi = wi;
-      out->pdf = ggx_d_visible(b.ggx, wo, h) / (4.0f * fmaxf(dot(wo, h), 1e-8f));
+      out->pdf = ggx_d_visible_from(b.wo_lam, ggx_d(b.ggx, h), wo, h) / (4.0f * fmaxf(dot(wo, h), 1e-8f));
       out->f = bsdf_eval<KM>(b, wo, wi);
       return true;
     }
     case B_COATED:
       if constexpr (!KM_HAS(KM, B_COATED)) return false;
-      return coated_sample(b.ggx, b.eta1, b.base, wo, u0, u1, u2, out);
+      return coated_sample(b, wo, u0, u1, u2, out);
     case B_DIFFUSE: {
       if constexpr (!KM_HAS(KM, B_DIFFUSE)) return false;
       if (wo.z <= 0.0f) return false;
@@ -311,10 +348,15 @@ __device__ bool bsdf_sample(const Bsdf& b, V3 wo, float u0, float u1, float u2, 
         V3 h = ggx_sample_h(b.ggx, wol, u1, u2);
         wi = to_world(fr, reflect(wol, h));
       } else {
+        // The body's coated lobe.
         BsdfSample s;
-        if (!coated_sample(ggx_from_roughness(0.12f), 1.45f, b.base, wo, (u0 - b.w) / fmaxf(1.0f - b.w, 1e-6f), u1, u2,
-                           &s))
-          return false;
+        Bsdf body;
+        body.kind = B_COATED;
+        body.ggx = ggx_from_roughness(0.12f);
+        body.eta1 = 1.45f;
+        body.base = b.base;
+        bsdf_prepare<(1u << B_COATED)>(body, wo);
+        if (!coated_sample(body, wo, (u0 - b.w) / fmaxf(1.0f - b.w, 1e-6f), u1, u2, &s)) return false;
         wi = s.wi;
       }
       if (wi.z <= 0.0f) return false;

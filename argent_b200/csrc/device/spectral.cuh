@@ -125,6 +125,41 @@ __device__ __forceinline__ float fresnel_dielectric(float cos_theta_i, float eta
   return 0.5f * (r_parl * r_parl + r_perp * r_perp);
 }
 
+// fresnel_dielectric for cos in (0, 1], for a light sample's value: both
+// reflectances over one denominator, inv_eta2 = 1 / eta^2 (a division instead
+// of three).
+__device__ __forceinline__ float fresnel_dielectric_nee(float c, float eta, float inv_eta2) {
+  c = fminf(c, 1.0f);
+  const float ct2 = __fmaf_rn(-__fmaf_rn(-c, c, 1.0f), inv_eta2, 1.0f);
+  if (ct2 <= 0.0f) return 1.0f;
+  const float ct = sqrtf(ct2);
+  const float d1 = __fmaf_rn(eta, c, ct), d2 = __fmaf_rn(eta, ct, c), m = d1 * d2;
+  const float n1 = __fmaf_rn(eta, c, -ct) * d2, n2 = __fmaf_rn(-eta, ct, c) * d1;
+  return 0.5f * __fmaf_rn(n1, n1, n2 * n2) / (m * m);
+}
+
+// Unpolarised conductor reflectance for cos in [0, 1] in real arithmetic, for
+// a light sample's value: with a + ib = sqrt((eta + ik)^2 - sin^2),
+// Rs = ((a - c)^2 + b^2) / ((a + c)^2 + b^2) and Rp = Rs ((ac - s)^2 + (bc)^2) /
+// ((ac + s)^2 + (bc)^2), s = sin^2 (Born and Wolf, Principles of Optics,
+// 14.2).  Of a and b the larger comes from the square root and the other from
+// ab = eta k, so neither cancels.  Two divisions where the complex quotients
+// take nine.
+__device__ __forceinline__ float fresnel_conductor_nee(float cos_theta, float eta, float k) {
+  const float c = rclamp(cos_theta, 0.0f, 1.0f);
+  const float s2 = 1.0f - c * c;
+  const float ek = eta * k;
+  const float t0 = __fmaf_rn(eta, eta, -(k * k)) - s2;
+  const float m = sqrtf(__fmaf_rn(t0, t0, 4.0f * (ek * ek)));
+  const float big = sqrtf(0.5f * (m + fabsf(t0)));
+  const float small = ek / fmaxf(big, 1e-18f);
+  const float a = t0 >= 0.0f ? big : small, b = t0 >= 0.0f ? small : big;
+  const float b2 = b * b, bc2 = b2 * (c * c), ac = a * c;
+  const float n1 = __fmaf_rn(a - c, a - c, b2), d1 = __fmaf_rn(a + c, a + c, b2);
+  const float n2 = __fmaf_rn(ac - s2, ac - s2, bc2), d2 = __fmaf_rn(ac + s2, ac + s2, bc2);
+  return 0.5f * n1 * (d2 + n2) / (d1 * d2);
+}
+
 // fresnel.rs:81-93: exact unpolarised conductor Fresnel, complex f32.
 __device__ __forceinline__ float fresnel_conductor1(float cos_theta_i, float eta, float k) {
   float cos_i = rclamp(cos_theta_i, 0.0f, 1.0f);
@@ -211,6 +246,11 @@ __device__ __forceinline__ float ggx_g2(Ggx g, V3 wo, V3 wi) {
 __device__ __forceinline__ float ggx_d_visible(Ggx g, V3 wo, V3 h) {
   float c = fmaxf(fabsf(wo.z), 1e-8f);
   return ggx_g1(g, wo) * fmaxf(dot(wo, h), 0.0f) * ggx_d(g, h) / c;
+}
+// ggx_d_visible from lambda of wo and D of h.
+__device__ __forceinline__ float ggx_d_visible_from(float lambda_wo, float d, V3 wo, V3 h) {
+  float c = fmaxf(fabsf(wo.z), 1e-8f);
+  return (1.0f / (1.0f + lambda_wo)) * fmaxf(dot(wo, h), 0.0f) * d / c;
 }
 __device__ __forceinline__ V3 ggx_sample_h(Ggx g, V3 wo, float u1, float u2) {
   float a = g.alpha;

@@ -881,10 +881,7 @@ __device__ __forceinline__ ShadeOut shade_path(const WaveArgs& a, uint32_t slot,
     s.draw<4>(set, ua);
     float ub = ua[0];
     Bsdf bsdf = material_bsdf<CLS>(mat, wl, cavity, ub, ctx);
-    if (bsdf.kind == B_CONDUCTOR && !is_smooth(bsdf.ggx)) {
-      bsdf.f0 = fresnel_conductor(1.0f, bsdf.eta, bsdf.k);
-      bsdf.e_wo = ggx_e(bsdf.ggx, wo.z);
-    }
+    bsdf_prepare<KM>(bsdf, wo);
     if (depth == 0) {
       float g[3];
       guide_rgb(mat, cavity, g);
@@ -947,7 +944,7 @@ __device__ __forceinline__ ShadeOut shade_path(const WaveArgs& a, uint32_t slot,
         V3 wi = to_local(frame, dir);
         Spec f;
         float p_bsdf;
-        bsdf_eval_pdf<KM>(bsdf, wo, wi, &f, &p_bsdf);
+        bsdf_nee<KM>(bsdf, wo, wi, &f, &p_bsdf);
         if (!is_black(f)) {
           float w = p_light * p_light / (p_light * p_light + p_bsdf * p_bsdf);
           // sky_visibility (scene.rs:123-140) for the map, visible
