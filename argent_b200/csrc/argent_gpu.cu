@@ -785,51 +785,50 @@ int argent_trace_anyhit(ArgentCtx* ctx, ArgentPiece* piece, const ArgentRay* ray
 
 namespace {
 
+// The filter's kernels for one set of guides; `sig` .. `vb` are its scratch.
+template <bool ALBEDO, bool NORMAL>
+void launch_atrous(ArgentCtx* ctx, uint32_t w, uint32_t h, const float* d_color, const float* d_albedo,
+                   const float* d_normal, float4* sig, float4* sig2, float4* guide, float2* nyz, float* va, float* vb,
+                   float* d_out) {
+  const uint32_t np = w * h;
+  cudaStream_t st = ctx->stream;
+  const int grid = std::max<int>(1, (int)std::min<uint32_t>((np + 255) / 256, (uint32_t)ctx->num_sms * 8));
+  const uint32_t tiles = (w + 31) / 32 * ((h + 7) / 8);
+  dn::k_dn_prep<ALBEDO, NORMAL><<<grid, 256, 0, st>>>(d_color, d_albedo, d_normal, np, sig, guide, nyz);
+  // noise_variance (denoise.rs:582-586)
+  dn::k_dn_resid<<<tiles, 256, 0, st>>>(sig, w, h, vb);
+  dn::k_dn_box5<<<tiles, 256, 0, st>>>(vb, va, w, h);
+  for (int pass = 0; pass + 1 < DN_PASSES; ++pass) {
+    dn::k_dn_atrous<ALBEDO, NORMAL, false><<<tiles, 256, 0, st>>>(sig, va, guide, nyz, w, h, 1 << pass, sig2, vb,
+                                                                 nullptr);
+    std::swap(sig, sig2);
+    std::swap(va, vb);
+  }
+  dn::k_dn_atrous<ALBEDO, NORMAL, true><<<tiles, 256, 0, st>>>(sig, va, guide, nyz, w, h, 1 << (DN_PASSES - 1),
+                                                              nullptr, nullptr, d_out);
+  ctx->launches += 3 + DN_PASSES;
+}
+
 // argent-post's atrous (denoise.rs:653-712) on device buffers: d_color
-// (and the optional guides) in, d_out out; w*h pixels, 3 floats each.
+// (and the optional guides; a normal only with an albedo) in, d_out out; w*h
+// pixels, 3 floats each.
 int run_atrous(ArgentCtx* ctx, uint32_t w, uint32_t h, const float* d_color, const float* d_albedo,
                const float* d_normal, float* d_out) {
   size_t np = (size_t)w * h;
   cudaStream_t st = ctx->stream;
   float* base = nullptr;
-  // sig, sig2, demod, g_albedo, g_normal (3 np each); l, l2, var, var2, vb, tmp, tmp2 (np each)
-  size_t total = 15 * np + 7 * np;
-  ARGENT_CK(ctx, cudaMallocAsync((void**)&base, total * sizeof(float), st));
-  float *sig = base, *sig2 = sig + 3 * np, *demod = sig2 + 3 * np, *ga = demod + 3 * np, *gn = ga + 3 * np;
-  float *l = gn + 3 * np, *l2 = l + np, *var = l2 + np, *var2 = var + np, *vb = var2 + np, *tmp = vb + np,
-        *tmp2 = tmp + np;
-  int grid = (int)std::min<size_t>((np + 255) / 256, (size_t)ctx->num_sms * 8);
-  grid = std::max(grid, 1);
-  auto blur = [&](const float* src, float* dst, std::initializer_list<float> k) {
-    dn::Taps t{};
-    t.n = 0;
-    for (float v : k) t.k[t.n++] = v;
-    dn::k_dn_blur<<<grid, 256, 0, st>>>(src, tmp2, w, h, t, 0);
-    dn::k_dn_blur<<<grid, 256, 0, st>>>(tmp2, dst, w, h, t, 1);
-    ctx->launches += 2;
-  };
-  dn::k_dn_prep<<<grid, 256, 0, st>>>(d_color, d_albedo, d_normal, (uint32_t)np, sig, l, demod, ga, gn);
-  ctx->launches++;
-  // noise_variance (denoise.rs:582-586)
-  blur(l, tmp, {1.0f, 1.0f, 1.0f});
-  dn::k_dn_resid<<<grid, 256, 0, st>>>(l, tmp, (uint32_t)np, vb);
-  ctx->launches++;
-  blur(vb, var, {1.0f, 1.0f, 1.0f, 1.0f, 1.0f});
-  for (int pass = 0; pass < DN_PASSES; ++pass) {
-    blur(var, vb, {0.25f, 0.5f, 0.25f});
-    dn::k_dn_atrous<<<grid, 256, 0, st>>>(sig, l, var, vb, d_albedo ? ga : nullptr, d_normal ? gn : nullptr, w, h,
-                                          1 << pass, sig2, var2, l2);
-    ctx->launches++;
-    std::swap(sig, sig2);
-    std::swap(var, var2);
-    std::swap(l, l2);
-  }
-  if (d_albedo) {
-    dn::k_dn_remod<<<grid, 256, 0, st>>>(sig, demod, (uint32_t)np);
-    ctx->launches++;
-  }
+  // sig, sig2, guide (4 np each), nyz (2 np), two variances (np each)
+  ARGENT_CK(ctx, cudaMallocAsync((void**)&base, 16 * np * sizeof(float), st));
+  float4 *sig = (float4*)base, *sig2 = sig + np, *guide = sig2 + np;
+  float2* nyz = (float2*)(guide + np);
+  float *va = (float*)(nyz + np), *vb = va + np;
+  if (d_albedo && d_normal)
+    launch_atrous<true, true>(ctx, w, h, d_color, d_albedo, d_normal, sig, sig2, guide, nyz, va, vb, d_out);
+  else if (d_albedo)
+    launch_atrous<true, false>(ctx, w, h, d_color, d_albedo, d_normal, sig, sig2, guide, nyz, va, vb, d_out);
+  else
+    launch_atrous<false, false>(ctx, w, h, d_color, d_albedo, d_normal, sig, sig2, guide, nyz, va, vb, d_out);
   cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaMemcpyAsync(d_out, sig, 3 * np * sizeof(float), cudaMemcpyDeviceToDevice, st);
   cudaFreeAsync(base, st);
   if (e != cudaSuccess) return set_error(ctx, ARGENT_E_CUDA, std::string("denoise: ") + cudaGetErrorString(e));
   return ARGENT_OK;
