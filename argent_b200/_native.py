@@ -193,6 +193,8 @@ GPU_FUNCS = {
                                                    ctypes.c_uint64, ctypes.c_void_p]),
     "argent_trace_anyhit_device": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                                                   ctypes.c_uint64, ctypes.c_void_p]),
+    "argent_pinned_alloc": (ctypes.c_int, [ctypes.c_size_t, ctypes.POINTER(ctypes.c_void_p)]),
+    "argent_pinned_free": (None, [ctypes.c_void_p]),
     "argent_render_batch": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ArgentBatchItem), ctypes.c_uint32]),
     "argent_autotune": (ctypes.c_int, [ctypes.c_void_p, ctypes.c_void_p, ctypes.POINTER(ArgentCamera),
                                        ctypes.POINTER(ArgentPathSettings), ctypes.c_uint32, ctypes.c_uint32,

@@ -193,10 +193,12 @@ __global__ void k_cavity_ao_finish(const uint32_t* counts, uint32_t nv, uint32_t
 
 // ------------------------------------------------------------------ context
 
+// Waits for the context stream and reports what its kernels recorded.
 int ctx_check_status(ArgentCtx* ctx) {
-  uint32_t st = 0;
-  ARGENT_CK(ctx, cudaMemcpyAsync(&st, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
+  ARGENT_CK(ctx,
+            cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
   ARGENT_CK(ctx, cudaStreamSynchronize(ctx->stream));
+  const uint32_t st = *ctx->h_status;
   if (st) {
     ARGENT_CK(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(uint32_t), ctx->stream));
     ARGENT_CK(ctx, cudaStreamSynchronize(ctx->stream));
@@ -207,6 +209,26 @@ int ctx_check_status(ArgentCtx* ctx) {
     return set_error(ctx, (st & ARGENT_STATUS_TIMEOUT) ? ARGENT_E_TIMEOUT : ARGENT_E_OVERFLOW, m);
   }
   return ARGENT_OK;
+}
+
+// Scratch of one call, on the context stream (freed with cudaFreeAsync).
+cudaError_t scratch_alloc(ArgentCtx* ctx, void** p, size_t bytes) {
+  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, ctx->scratch, ctx->stream);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  cudaStreamSynchronize(ctx->stream);
+  cudaMemPoolTrimTo(ctx->scratch, 0);
+  return cudaMallocFromPoolAsync(p, bytes, ctx->scratch, ctx->stream);
+}
+
+// Device memory of an object; the kept scratch gives way when it runs out.
+cudaError_t device_alloc(ArgentCtx* ctx, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  cudaStreamSynchronize(ctx->stream);
+  cudaMemPoolTrimTo(ctx->scratch, 0);
+  return cudaMalloc(p, bytes);
 }
 
 int grid_for(const ArgentCtx* ctx, const void* kernel, int block, uint64_t n) {
@@ -311,6 +333,18 @@ int argent_ctx_create(int device, const ArgentLimits* limits, ArgentCtx** out) {
   if (r == cudaSuccess) r = cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
   if (r == cudaSuccess) r = cudaMalloc(&ctx->d_status, sizeof(uint32_t) * 4);
   if (r == cudaSuccess) r = cudaMemset(ctx->d_status, 0, sizeof(uint32_t) * 4);
+  if (r == cudaSuccess) r = cudaMallocHost((void**)&ctx->h_status, 4096);
+  if (r == cudaSuccess) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    r = cudaMemPoolCreate(&ctx->scratch, &props);
+  }
+  if (r == cudaSuccess) {
+    uint64_t keep = ARGENT_SCRATCH_KEEP;
+    r = cudaMemPoolSetAttribute(ctx->scratch, cudaMemPoolAttrReleaseThreshold, &keep);
+  }
   if (r != cudaSuccess) {
     std::string m = std::string("context setup failed: ") + cudaGetErrorString(r);
     argent_ctx_destroy(ctx);
@@ -338,6 +372,8 @@ void argent_ctx_destroy(ArgentCtx* ctx) {
   for (auto& b : ctx->blobs) cudaFree(b.dev);
   ctx->blobs.clear();
   if (ctx->d_status) cudaFree(ctx->d_status);
+  if (ctx->h_status) cudaFreeHost(ctx->h_status);
+  if (ctx->scratch) cudaMemPoolDestroy(ctx->scratch);
   if (ctx->resolve) cudaFree(ctx->resolve);
   if (ctx->d_jobs_buf) cudaFree(ctx->d_jobs_buf);
   for (auto& g : ctx->graph_cache) cudaGraphExecDestroy(g.exec);
@@ -366,6 +402,20 @@ int argent_ctx_sync(ArgentCtx* ctx) {
   if (ctx->aux_stream) ARGENT_CK(ctx, cudaStreamSynchronize(ctx->aux_stream));
   ctx->overlapped_pending = false;
   return ctx_check_status(ctx);
+}
+
+int argent_pinned_alloc(size_t bytes, void** out) {
+  if (!out || bytes == 0) return set_error(nullptr, ARGENT_E_INVALID, "argent_pinned_alloc: NULL argument or no bytes");
+  *out = nullptr;
+  cudaError_t e = cudaHostAlloc(out, bytes, cudaHostAllocPortable);
+  if (e == cudaSuccess) return ARGENT_OK;
+  cudaGetLastError();
+  return set_error(nullptr, e == cudaErrorMemoryAllocation ? ARGENT_E_OOM : ARGENT_E_CUDA,
+                   std::string("argent_pinned_alloc: ") + cudaGetErrorString(e));
+}
+
+void argent_pinned_free(void* p) {
+  if (p) cudaFreeHost(p);
 }
 
 void* argent_ctx_stream(ArgentCtx* ctx) { return ctx ? (void*)ctx->stream : nullptr; }
@@ -419,7 +469,7 @@ int argent_piece_upload(ArgentCtx* ctx, const float* positions, uint32_t nv, con
   auto up = [&](const void* src, size_t bytes, void** dst) -> cudaError_t {
     *dst = nullptr;
     if (bytes == 0) return cudaSuccess;
-    cudaError_t e = cudaMalloc(dst, bytes);
+    cudaError_t e = device_alloc(ctx, (void**)dst, bytes);
     if (e != cudaSuccess) return e;
     p->allocs.push_back(*dst);
     p->bytes += bytes;
@@ -455,13 +505,14 @@ namespace {
 
 // Stream-ordered temporaries of one device build, freed together.
 struct BuildTemps {
+  ArgentCtx* ctx;
   cudaStream_t st;
   std::vector<void*> ptrs;
   cudaError_t err = cudaSuccess;
   template <class T>
   T* get(size_t count) {
     void* p = nullptr;
-    if (err == cudaSuccess) err = cudaMallocAsync(&p, std::max<size_t>(count, 1) * sizeof(T), st);
+    if (err == cudaSuccess) err = scratch_alloc(ctx, &p, std::max<size_t>(count, 1) * sizeof(T));
     if (err == cudaSuccess) ptrs.push_back(p);
     return (T*)p;
   }
@@ -476,7 +527,7 @@ struct BuildTemps {
 std::string device_bvh(ArgentCtx* ctx, ArgentPiece* p, const float4* pos, const uint4* tidx, uint32_t nt) {
   cudaStream_t st = ctx->stream;
   const size_t n = nt, nb = 2 * n - 1;
-  BuildTemps tmp{st};
+  BuildTemps tmp{ctx, st};
   const uint32_t tpb = 256;
   const uint32_t nblk = (uint32_t)std::min<size_t>((n + tpb - 1) / tpb, (size_t)148 * 8);
   float* tlo = tmp.get<float>(3 * n);
@@ -505,7 +556,7 @@ std::string device_bvh(ArgentCtx* ctx, ArgentPiece* p, const float4* pos, const 
   if (tmp.err != cudaSuccess) return std::string("device BVH temporaries: ") + cudaGetErrorString(tmp.err);
 
   void* dt = nullptr;
-  cudaError_t e = cudaMalloc(&dt, n * sizeof(argent::TriRecord));
+  cudaError_t e = device_alloc(ctx, (void**)&dt, n * sizeof(argent::TriRecord));
   if (e != cudaSuccess) return std::string("device BVH triangles: ") + cudaGetErrorString(e);
   p->allocs.push_back(dt);
   p->bytes += n * sizeof(argent::TriRecord);
@@ -572,7 +623,7 @@ std::string device_bvh(ArgentCtx* ctx, ArgentPiece* p, const float4* pos, const 
 
   void* dn = nullptr;
   const size_t node_bytes = (size_t)got[1] * sizeof(argent::WideNode);
-  e = cudaMalloc(&dn, node_bytes);
+  e = device_alloc(ctx, (void**)&dn, node_bytes);
   if (e != cudaSuccess) return std::string("device BVH nodes: ") + cudaGetErrorString(e);
   p->allocs.push_back(dn);
   p->bytes += node_bytes;
@@ -624,7 +675,7 @@ int argent_piece_upload_device_bvh(ArgentCtx* ctx, const float* positions, uint3
   auto up = [&](const void* src, size_t bytes, void** dst) -> cudaError_t {
     *dst = nullptr;
     if (bytes == 0) return cudaSuccess;
-    cudaError_t e = cudaMalloc(dst, bytes);
+    cudaError_t e = device_alloc(ctx, (void**)dst, bytes);
     if (e != cudaSuccess) return e;
     p->allocs.push_back(*dst);
     p->bytes += bytes;
@@ -735,8 +786,8 @@ int argent_trace_closest(ArgentCtx* ctx, ArgentPiece* piece, const ArgentRay* ra
   if (n == 0) return ARGENT_OK;
   ARGENT_CK(ctx, cudaSetDevice(ctx->device));
   void *dr = nullptr, *dh = nullptr;
-  ARGENT_CK(ctx, cudaMallocAsync(&dr, n * sizeof(ArgentRay), ctx->stream));
-  cudaError_t e = cudaMallocAsync(&dh, n * sizeof(ArgentHit), ctx->stream);
+  ARGENT_CK(ctx, scratch_alloc(ctx, (void**)&dr, n * sizeof(ArgentRay)));
+  cudaError_t e = scratch_alloc(ctx, (void**)&dh, n * sizeof(ArgentHit));
   if (e != cudaSuccess) {
     cudaFreeAsync(dr, ctx->stream);
     return set_error(ctx, ARGENT_E_OOM, "trace buffers");
@@ -748,8 +799,7 @@ int argent_trace_closest(ArgentCtx* ctx, ArgentPiece* piece, const ArgentRay* ra
     e = cudaMemcpyAsync(hits, dh, n * sizeof(ArgentHit), cudaMemcpyDeviceToHost, ctx->stream);
   cudaFreeAsync(dr, ctx->stream);
   cudaFreeAsync(dh, ctx->stream);
-  cudaError_t s = cudaStreamSynchronize(ctx->stream);
-  if (e == cudaSuccess) e = s;
+  if (rc != ARGENT_OK || e != cudaSuccess) cudaStreamSynchronize(ctx->stream);
   if (rc != ARGENT_OK) return rc;
   if (e != cudaSuccess) return set_error(ctx, ARGENT_E_CUDA, std::string("trace: ") + cudaGetErrorString(e));
   return ctx_check_status(ctx);
@@ -760,8 +810,8 @@ int argent_trace_anyhit(ArgentCtx* ctx, ArgentPiece* piece, const ArgentRay* ray
   if (n == 0) return ARGENT_OK;
   ARGENT_CK(ctx, cudaSetDevice(ctx->device));
   void *dr = nullptr, *dh = nullptr;
-  ARGENT_CK(ctx, cudaMallocAsync(&dr, n * sizeof(ArgentRay), ctx->stream));
-  cudaError_t e = cudaMallocAsync(&dh, n, ctx->stream);
+  ARGENT_CK(ctx, scratch_alloc(ctx, (void**)&dr, n * sizeof(ArgentRay)));
+  cudaError_t e = scratch_alloc(ctx, (void**)&dh, n);
   if (e != cudaSuccess) {
     cudaFreeAsync(dr, ctx->stream);
     return set_error(ctx, ARGENT_E_OOM, "trace buffers");
@@ -772,8 +822,7 @@ int argent_trace_anyhit(ArgentCtx* ctx, ArgentPiece* piece, const ArgentRay* ray
   if (e == cudaSuccess && rc == ARGENT_OK) e = cudaMemcpyAsync(occluded, dh, n, cudaMemcpyDeviceToHost, ctx->stream);
   cudaFreeAsync(dr, ctx->stream);
   cudaFreeAsync(dh, ctx->stream);
-  cudaError_t s = cudaStreamSynchronize(ctx->stream);
-  if (e == cudaSuccess) e = s;
+  if (rc != ARGENT_OK || e != cudaSuccess) cudaStreamSynchronize(ctx->stream);
   if (rc != ARGENT_OK) return rc;
   if (e != cudaSuccess) return set_error(ctx, ARGENT_E_CUDA, std::string("trace: ") + cudaGetErrorString(e));
   return ctx_check_status(ctx);
@@ -818,7 +867,7 @@ int run_atrous(ArgentCtx* ctx, uint32_t w, uint32_t h, const float* d_color, con
   cudaStream_t st = ctx->stream;
   float* base = nullptr;
   // sig, sig2, guide (4 np each), nyz (2 np), two variances (np each)
-  ARGENT_CK(ctx, cudaMallocAsync((void**)&base, 16 * np * sizeof(float), st));
+  ARGENT_CK(ctx, scratch_alloc(ctx, (void**)&base, 16 * np * sizeof(float)));
   float4 *sig = (float4*)base, *sig2 = sig + np, *guide = sig2 + np;
   float2* nyz = (float2*)(guide + np);
   float *va = (float*)(nyz + np), *vb = va + np;
@@ -847,7 +896,7 @@ int argent_denoise_atrous(ArgentCtx* ctx, uint32_t width, uint32_t height, const
   if (np > (1ull << 31)) return set_error(ctx, ARGENT_E_INVALID, "image too large");
   ARGENT_CK(ctx, cudaSetDevice(ctx->device));
   float* d = nullptr;
-  ARGENT_CK(ctx, cudaMallocAsync((void**)&d, 12 * np * sizeof(float), ctx->stream));
+  ARGENT_CK(ctx, scratch_alloc(ctx, (void**)&d, 12 * np * sizeof(float)));
   float *dc = d, *da = albedo ? d + 3 * np : nullptr, *dn_ = normal ? d + 6 * np : nullptr, *dout = d + 9 * np;
   cudaError_t e = cudaMemcpyAsync(dc, color, 3 * np * sizeof(float), cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess && da) e = cudaMemcpyAsync(da, albedo, 3 * np * sizeof(float), cudaMemcpyHostToDevice, ctx->stream);
@@ -855,7 +904,7 @@ int argent_denoise_atrous(ArgentCtx* ctx, uint32_t width, uint32_t height, const
   int rc = e == cudaSuccess ? run_atrous(ctx, width, height, dc, da, dn_, dout) : ARGENT_E_CUDA;
   if (rc == ARGENT_OK) e = cudaMemcpyAsync(out, dout, 3 * np * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream);
   cudaFreeAsync(d, ctx->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  if (rc != ARGENT_OK || e != cudaSuccess) cudaStreamSynchronize(ctx->stream);
   if (rc != ARGENT_OK) return rc;
   if (e != cudaSuccess) return set_error(ctx, ARGENT_E_CUDA, std::string("denoise: ") + cudaGetErrorString(e));
   return ctx_check_status(ctx);
@@ -876,7 +925,7 @@ int run_develop(ArgentCtx* ctx, uint32_t w, uint32_t h, const float* d_rgb, cons
   argent::DevelopTables t = argent::develop_tables(g->exposure_ev, g->tonemap, g->look, g->saturation);
   size_t nc = t.curves.size(), ne = t.enc.size();
   float* d_tab = nullptr;
-  ARGENT_CK(ctx, cudaMallocAsync((void**)&d_tab, (nc + ne) * sizeof(float), ctx->stream));
+  ARGENT_CK(ctx, scratch_alloc(ctx, (void**)&d_tab, (nc + ne) * sizeof(float)));
   cudaError_t e = cudaSuccess;
   if (nc) e = cudaMemcpyAsync(d_tab, t.curves.data(), nc * sizeof(float), cudaMemcpyHostToDevice, ctx->stream);
   if (e == cudaSuccess)
@@ -920,14 +969,14 @@ int argent_develop(ArgentCtx* ctx, uint32_t width, uint32_t height, const float*
   ARGENT_CK(ctx, cudaSetDevice(ctx->device));
   float* d_rgb = nullptr;
   uint8_t* d_out = nullptr;
-  ARGENT_CK(ctx, cudaMallocAsync((void**)&d_rgb, 3 * np * sizeof(float), ctx->stream));
-  ARGENT_CK(ctx, cudaMallocAsync((void**)&d_out, 3 * np, ctx->stream));
+  ARGENT_CK(ctx, scratch_alloc(ctx, (void**)&d_rgb, 3 * np * sizeof(float)));
+  ARGENT_CK(ctx, scratch_alloc(ctx, (void**)&d_out, 3 * np));
   cudaError_t e = cudaMemcpyAsync(d_rgb, rgb, 3 * np * sizeof(float), cudaMemcpyHostToDevice, ctx->stream);
   int rc = e == cudaSuccess ? run_develop(ctx, width, height, d_rgb, grade, d_out) : ARGENT_E_CUDA;
   if (rc == ARGENT_OK) e = cudaMemcpyAsync(out, d_out, 3 * np, cudaMemcpyDeviceToHost, ctx->stream);
   cudaFreeAsync(d_rgb, ctx->stream);
   cudaFreeAsync(d_out, ctx->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  if (rc != ARGENT_OK || e != cudaSuccess) cudaStreamSynchronize(ctx->stream);
   if (rc != ARGENT_OK) return rc;
   if (e != cudaSuccess) return set_error(ctx, ARGENT_E_CUDA, std::string("develop: ") + cudaGetErrorString(e));
   return ctx_check_status(ctx);
@@ -990,9 +1039,9 @@ int argent_piece_ambient_occlusion(ArgentCtx* ctx, ArgentPiece* piece, const flo
   float* d_n = nullptr;
   uint32_t* d_cnt = nullptr;
   float* d_ao = nullptr;
-  ARGENT_CK(ctx, cudaMallocAsync((void**)&d_n, 3ull * nv * sizeof(float), ctx->stream));
-  ARGENT_CK(ctx, cudaMallocAsync((void**)&d_cnt, (size_t)nv * sizeof(uint32_t), ctx->stream));
-  ARGENT_CK(ctx, cudaMallocAsync((void**)&d_ao, (size_t)nv * sizeof(float), ctx->stream));
+  ARGENT_CK(ctx, scratch_alloc(ctx, (void**)&d_n, 3ull * nv * sizeof(float)));
+  ARGENT_CK(ctx, scratch_alloc(ctx, (void**)&d_cnt, (size_t)nv * sizeof(uint32_t)));
+  ARGENT_CK(ctx, scratch_alloc(ctx, (void**)&d_ao, (size_t)nv * sizeof(float)));
   ARGENT_CK(ctx, cudaMemcpyAsync(d_n, normals, 3ull * nv * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
   ARGENT_CK(ctx, cudaMemsetAsync(d_cnt, 0, (size_t)nv * sizeof(uint32_t), ctx->stream));
   uint64_t total = (uint64_t)nv * samples;
@@ -1010,7 +1059,7 @@ int argent_piece_ambient_occlusion(ArgentCtx* ctx, ArgentPiece* piece, const flo
   cudaFreeAsync(d_n, ctx->stream);
   cudaFreeAsync(d_cnt, ctx->stream);
   cudaFreeAsync(d_ao, ctx->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  if (e != cudaSuccess) cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) return set_error(ctx, ARGENT_E_CUDA, std::string("ambient occlusion: ") + cudaGetErrorString(e));
   return ctx_check_status(ctx);
 }
@@ -1100,7 +1149,7 @@ static int ensure_wave(ArgentCtx* ctx, int lane, uint64_t cap) {
   if (w.cap > 0) ARGENT_CK(ctx, cudaStreamSynchronize(ctx->lane_stream[lane]));
   w.release();
   auto alloc = [&](void** p, size_t bytes) -> bool {
-    if (cudaMalloc(p, bytes) != cudaSuccess) return false;
+    if (device_alloc(ctx, (void**)p, bytes) != cudaSuccess) return false;
     w.allocs.push_back(*p);
     w.bytes += bytes;
     return true;
@@ -1129,7 +1178,7 @@ static int ensure_share(ArgentCtx* ctx, int lane, uint64_t cap) {
   if (w.share_cap > 0) ARGENT_CK(ctx, cudaStreamSynchronize(ctx->lane_stream[lane]));
   w.release_share();
   auto alloc = [&](void** p, size_t bytes) -> bool {
-    if (cudaMalloc(p, bytes) != cudaSuccess) return false;
+    if (device_alloc(ctx, (void**)p, bytes) != cudaSuccess) return false;
     w.share_allocs.push_back(*p);
     w.share_bytes += bytes;
     w.bytes += bytes;
@@ -1454,13 +1503,13 @@ static int run_jobs(ArgentCtx* ctx, const std::vector<dev::DevJob>& jobs, const 
       ctx->d_jobs_buf = nullptr;
       ctx->d_jobs_cap = 0;
       size_t n = std::max<size_t>(jobs.size(), 64);
-      if (cudaMalloc((void**)&ctx->d_jobs_buf, n * sizeof(dev::DevJob)) != cudaSuccess)
+      if (device_alloc(ctx, (void**)&ctx->d_jobs_buf, n * sizeof(dev::DevJob)) != cudaSuccess)
         return set_error(ctx, ARGENT_E_OOM, "job records: out of device memory");
       ctx->d_jobs_cap = n;
     }
     d_jobs = ctx->d_jobs_buf;
   } else {
-    ARGENT_CK(ctx, cudaMallocAsync((void**)&d_jobs, jobs.size() * sizeof(dev::DevJob), ctx->stream));
+    ARGENT_CK(ctx, scratch_alloc(ctx, (void**)&d_jobs, jobs.size() * sizeof(dev::DevJob)));
   }
   // Pageable source: the call returns once the bytes are staged.
   ARGENT_CK(ctx, cudaMemcpyAsync(d_jobs, job_list->data(), jobs.size() * sizeof(dev::DevJob), cudaMemcpyHostToDevice,
@@ -1841,7 +1890,7 @@ static void* intern_blob(ArgentCtx* ctx, const void* src, size_t bytes, std::vec
     }
   }
   ArgentCtx::SharedBlob b;
-  if (cudaMalloc(&b.dev, bytes) != cudaSuccess) return nullptr;
+  if (device_alloc(ctx, (void**)&b.dev, bytes) != cudaSuccess) return nullptr;
   if (cudaMemcpy(b.dev, src, bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
     cudaFree(b.dev);
     return nullptr;
@@ -1921,7 +1970,7 @@ int argent_scene_upload(ArgentCtx* ctx, ArgentPiece* piece, const ArgentSceneDes
   h.piece = piece->dev;
   auto up = [&](const void* src, size_t bytes) -> void* {
     void* d = nullptr;
-    if (cudaMalloc(&d, bytes) != cudaSuccess) return nullptr;
+    if (device_alloc(ctx, (void**)&d, bytes) != cudaSuccess) return nullptr;
     s->allocs.push_back(d);
     s->bytes += bytes;
     if (cudaMemcpy(d, src, bytes, cudaMemcpyHostToDevice) != cudaSuccess) return nullptr;
@@ -2064,11 +2113,11 @@ int argent_film_create(ArgentCtx* ctx, uint32_t width, uint32_t height, uint32_t
   f->h = height;
   f->flags = flags;
   size_t n = 3ull * width * height;
-  bool ok = cudaMalloc(&f->xyz, n * sizeof(float)) == cudaSuccess;
-  ok = ok && cudaMalloc(&f->albedo, n * sizeof(float)) == cudaSuccess;
-  ok = ok && cudaMalloc(&f->normal, n * sizeof(float)) == cudaSuccess;
-  if (ok && (flags & ARGENT_FILM_KAHAN)) ok = cudaMalloc(&f->comp, n * sizeof(float)) == cudaSuccess;
-  if (ok && (flags & ARGENT_FILM_FP64)) ok = cudaMalloc(&f->xyz64, n * sizeof(double)) == cudaSuccess;
+  bool ok = device_alloc(ctx, (void**)&f->xyz, n * sizeof(float)) == cudaSuccess;
+  ok = ok && device_alloc(ctx, (void**)&f->albedo, n * sizeof(float)) == cudaSuccess;
+  ok = ok && device_alloc(ctx, (void**)&f->normal, n * sizeof(float)) == cudaSuccess;
+  if (ok && (flags & ARGENT_FILM_KAHAN)) ok = device_alloc(ctx, (void**)&f->comp, n * sizeof(float)) == cudaSuccess;
+  if (ok && (flags & ARGENT_FILM_FP64)) ok = device_alloc(ctx, (void**)&f->xyz64, n * sizeof(double)) == cudaSuccess;
   if (!ok) {
     argent_film_destroy(f);
     return set_error(ctx, ARGENT_E_OOM, "film: out of device memory");
@@ -2179,7 +2228,7 @@ int ensure_resolve(ArgentCtx* ctx, size_t floats) {
   if (ctx->resolve) cudaFree(ctx->resolve);
   ctx->resolve = nullptr;
   ctx->resolve_floats = 0;
-  if (cudaMalloc(&ctx->resolve, floats * sizeof(float)) != cudaSuccess)
+  if (device_alloc(ctx, (void**)&ctx->resolve, floats * sizeof(float)) != cudaSuccess)
     return set_error(ctx, ARGENT_E_OOM, "film read staging: out of device memory");
   ctx->resolve_floats = floats;
   return ARGENT_OK;
@@ -2217,7 +2266,6 @@ int argent_film_read(ArgentFilm* f, float* color, float* albedo, float* normal) 
     ARGENT_CK(ctx, cudaMemcpyAsync(albedo, d_albedo, 3 * np * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
   if (normal)
     ARGENT_CK(ctx, cudaMemcpyAsync(normal, d_normal, 3 * np * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
-  ARGENT_CK(ctx, cudaStreamSynchronize(ctx->stream));
   return ctx_check_status(ctx);
 }
 
@@ -2240,12 +2288,12 @@ int argent_film_denoise(ArgentFilm* f, float* out) {
                                                               (uint32_t)np, dc, da, dnrm);
   ctx->launches++;
   float* dout = nullptr;
-  ARGENT_CK(ctx, cudaMallocAsync((void**)&dout, 3 * np * sizeof(float), ctx->stream));
+  ARGENT_CK(ctx, scratch_alloc(ctx, (void**)&dout, 3 * np * sizeof(float)));
   rc = run_atrous(ctx, f->w, f->h, dc, da, dnrm, dout);
   cudaError_t e = cudaSuccess;
   if (rc == ARGENT_OK) e = cudaMemcpyAsync(out, dout, 3 * np * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream);
   cudaFreeAsync(dout, ctx->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  if (rc != ARGENT_OK || e != cudaSuccess) cudaStreamSynchronize(ctx->stream);
   if (rc != ARGENT_OK) return rc;
   if (e != cudaSuccess) return set_error(ctx, ARGENT_E_CUDA, std::string("film denoise: ") + cudaGetErrorString(e));
   return ctx_check_status(ctx);
@@ -2272,8 +2320,8 @@ int argent_film_develop(ArgentFilm* f, const ArgentGrade* grade, int denoise, ui
   ctx->launches++;
   float* dd = nullptr;
   uint8_t* d8 = nullptr;
-  ARGENT_CK(ctx, cudaMallocAsync((void**)&dd, 3 * np * sizeof(float), ctx->stream));
-  ARGENT_CK(ctx, cudaMallocAsync((void**)&d8, 3 * np, ctx->stream));
+  ARGENT_CK(ctx, scratch_alloc(ctx, (void**)&dd, 3 * np * sizeof(float)));
+  ARGENT_CK(ctx, scratch_alloc(ctx, (void**)&d8, 3 * np));
   const float* src = dc;
   if (denoise) {
     rc = run_atrous(ctx, f->w, f->h, dc, da, dnrm, dd);
@@ -2284,7 +2332,7 @@ int argent_film_develop(ArgentFilm* f, const ArgentGrade* grade, int denoise, ui
   if (rc == ARGENT_OK) e = cudaMemcpyAsync(out, d8, 3 * np, cudaMemcpyDeviceToHost, ctx->stream);
   cudaFreeAsync(dd, ctx->stream);
   cudaFreeAsync(d8, ctx->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  if (rc != ARGENT_OK || e != cudaSuccess) cudaStreamSynchronize(ctx->stream);
   if (rc != ARGENT_OK) return rc;
   if (e != cudaSuccess) return set_error(ctx, ARGENT_E_CUDA, std::string("film develop: ") + cudaGetErrorString(e));
   return ctx_check_status(ctx);
@@ -2304,7 +2352,7 @@ static int promote_if_long(ArgentFilm* f, uint64_t end_samples) {
   if (!(f->flags & ARGENT_FILM_PROGRESSIVE) || f->xyz64 || end_samples <= ARGENT_FILM_FP64_AFTER) return ARGENT_OK;
   ArgentCtx* ctx = f->ctx;
   size_t n = 3ull * f->w * f->h;
-  cudaError_t e = cudaMalloc(&f->xyz64, n * sizeof(double));
+  cudaError_t e = device_alloc(ctx, (void**)&f->xyz64, n * sizeof(double));
   if (e != cudaSuccess) {
     f->xyz64 = nullptr;
     return set_error(ctx, ARGENT_E_OOM, "film: out of device memory for the FP64 sums");
@@ -2778,6 +2826,5 @@ extern "C" int argent_trace_closest_noalloc(ArgentCtx* ctx, ArgentPiece* piece, 
   ctx->launches++;
   ARGENT_CK(ctx, cudaGetLastError());
   ARGENT_CK(ctx, cudaMemcpyAsync(hits, d_hits, n * sizeof(ArgentHit), cudaMemcpyDeviceToHost, ctx->stream));
-  ARGENT_CK(ctx, cudaStreamSynchronize(ctx->stream));
   return ctx_check_status(ctx);
 }

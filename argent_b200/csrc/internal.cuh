@@ -186,6 +186,7 @@ struct KernelProfile {
 #define ARGENT_LANES 16
 #define ARGENT_GRAPH_CACHE 8
 #define ARGENT_SIDES 4
+#define ARGENT_SCRATCH_KEEP (1ull << 30)
 
 struct ArgentCtx {
   int device = 0;
@@ -249,6 +250,13 @@ struct ArgentCtx {
   std::string err;
   uint64_t launches = 0;
   uint32_t* d_status = nullptr;
+  uint32_t* h_status = nullptr;  // page-locked words for small reads: the status, a build's counters
+  // Stream-ordered scratch of single calls (rays and hits, images, build
+  // temporaries): up to ARGENT_SCRATCH_KEEP bytes stay with the context between
+  // calls.  The device's default pool gives everything back at each
+  // synchronisation, so every call mapped and unmapped its memory anew (0.4 of
+  // the 0.5 ms of an eight-ray trace; milliseconds for a full frame).
+  cudaMemPool_t scratch = nullptr;
   bool tables_ready = false;
   WaveBuffers wave[ARGENT_LANES];
   KernelProfile prof;
@@ -304,4 +312,6 @@ struct ArgentFilm {
 
 int set_error(const ArgentCtx* ctx, int code, const std::string& msg);
 int ctx_check_status(ArgentCtx* ctx);
+cudaError_t scratch_alloc(ArgentCtx* ctx, void** p, size_t bytes);
+cudaError_t device_alloc(ArgentCtx* ctx, void** p, size_t bytes);
 int grid_for(const ArgentCtx* ctx, const void* kernel, int block, uint64_t n);

@@ -6,6 +6,8 @@ These mirror argent's own objects: `Piece` (scene.rs:10-38), `Scene`
 """
 
 import ctypes
+import threading
+import weakref
 
 import numpy as np
 
@@ -16,6 +18,88 @@ def _p(a, t=ctypes.c_void_p):
     if a is None:
         return None
     return a.ctypes.data_as(t)
+
+
+class ResultPool:
+    """Arrays for results, in page-locked memory that is used again.
+
+    A result copied into fresh pageable memory pays for the driver's staging
+    copy and for the first touch of every page: a 1920 x 1080 film's three
+    images took 15 ms of a 300 ms render, and take 1.5 ms into page-locked
+    memory.  A block goes back to the pool once no array refers to it any more
+    (any thread may drop the last one).  At most LIMIT bytes are page-locked in
+    all; results beyond that, and those under SMALL bytes, are ordinary arrays.
+    At most IDLE bytes wait unused, the rest is freed."""
+
+    SMALL = 1 << 16
+    LIMIT = 1 << 30
+    IDLE = 1 << 29
+
+    def __init__(self):
+        # Reentrant: the garbage collector may finalise an array, and so
+        # return its block, while this thread holds the lock.
+        self._lock = threading.RLock()
+        self._free = {}  # block size -> addresses
+        self.total = 0  # bytes page-locked
+        self.idle = 0  # of these, waiting
+
+    @staticmethod
+    def _block(n):
+        """Block size of an n-byte result: the next eighth of a power of two,
+        so that nearby sizes share blocks."""
+        step = 1 << max(n.bit_length() - 4, 12)
+        return (n + step - 1) // step * step
+
+    def array(self, shape, dtype):
+        """An uninitialised array; its caller fills all of it."""
+        dtype = np.dtype(dtype)
+        count = int(np.prod(shape))
+        n = count * dtype.itemsize
+        if n < self.SMALL:
+            return np.empty(shape, dtype)
+        size = self._block(n)
+        ptr = None
+        with self._lock:
+            if self._free.get(size):
+                ptr = self._free[size].pop()
+                self.idle -= size
+            else:
+                self._trim(size)
+                if self.total + size > self.LIMIT:
+                    return np.empty(shape, dtype)
+                self.total += size
+        if ptr is None:
+            p = ctypes.c_void_p()
+            if N.gpu().argent_pinned_alloc(size, ctypes.byref(p)) != N.OK:
+                with self._lock:
+                    self.total -= size
+                return np.empty(shape, dtype)
+            ptr = p.value
+        buf = (ctypes.c_char * size).from_address(ptr)
+        weakref.finalize(buf, self._give, ptr, size).atexit = False
+        return np.frombuffer(buf, dtype, count).reshape(shape)
+
+    def _trim(self, size):
+        """Frees waiting blocks of other sizes until `size` more bytes fit."""
+        for k in sorted(self._free):
+            while self._free[k] and self.total + size > self.LIMIT:
+                self._release(self._free[k].pop(), k)
+                self.idle -= k
+
+    def _release(self, ptr, size):
+        N.gpu().argent_pinned_free(ptr)
+        self.total -= size
+
+    def _give(self, ptr, size):
+        with self._lock:
+            if self.idle + size > self.IDLE:
+                self._release(ptr, size)
+            else:
+                self._free.setdefault(size, []).append(ptr)
+                self.idle += size
+
+
+_results = ResultPool()
 
 
 class Context:
@@ -201,7 +285,7 @@ class Piece:
         m = self.mesh
         fp = ctypes.POINTER(ctypes.c_float)
         n = np.ascontiguousarray(normals, np.float32)
-        out = np.zeros(len(m.positions), np.float32)
+        out = _results.array(len(m.positions), np.float32)
         self.ctx.check(self.ctx.lib.argent_piece_ambient_occlusion(
             self.ctx.h, self.h, _p(m.positions, fp), _p(n, fp), len(m.positions), samples, distance, _p(out, fp)))
         return out
@@ -227,13 +311,13 @@ class Piece:
         """rays: (n, 8) float32 [ox oy oz tmax dx dy dz pad] -> hits (n, 4)
         float32 [t u v prim-bits]."""
         rays = np.ascontiguousarray(rays, np.float32)
-        hits = np.zeros((len(rays), 4), np.float32)
+        hits = _results.array((len(rays), 4), np.float32)
         self.ctx.check(self.ctx.lib.argent_trace_closest(self.ctx.h, self.h, _p(rays), len(rays), _p(hits)))
         return hits
 
     def trace_anyhit(self, rays: np.ndarray) -> np.ndarray:
         rays = np.ascontiguousarray(rays, np.float32)
-        occ = np.zeros(len(rays), np.uint8)
+        occ = _results.array(len(rays), np.uint8)
         self.ctx.check(self.ctx.lib.argent_trace_anyhit(self.ctx.h, self.h, _p(rays), len(rays), _p(occ)))
         return occ
 
@@ -291,14 +375,14 @@ class Film:
     def read(self):
         """(color, albedo, normal) as `Film::color/albedo/normal`, (h, w, 3)."""
         shape = (self.height, self.width, 3)
-        c, a, n = np.zeros(shape, np.float32), np.zeros(shape, np.float32), np.zeros(shape, np.float32)
+        c, a, n = (_results.array(shape, np.float32) for _ in range(3))
         fp = ctypes.POINTER(ctypes.c_float)
         self.ctx.check(self.ctx.lib.argent_film_read(self.h, _p(c, fp), _p(a, fp), _p(n, fp)))
         return c, a, n
 
     def color(self):
         shape = (self.height, self.width, 3)
-        c = np.zeros(shape, np.float32)
+        c = _results.array(shape, np.float32)
         fp = ctypes.POINTER(ctypes.c_float)
         self.ctx.check(self.ctx.lib.argent_film_read(self.h, _p(c, fp), None, None))
         return c
@@ -306,7 +390,7 @@ class Film:
     def denoised(self):
         """The colour denoised on the device with the film's albedo and
         normal guides (argent-post's à-trous backend)."""
-        out = np.zeros((self.height, self.width, 3), np.float32)
+        out = _results.array((self.height, self.width, 3), np.float32)
         self.ctx.check(self.ctx.lib.argent_film_denoise(self.h, _p(out, ctypes.POINTER(ctypes.c_float))))
         return out
 
@@ -314,7 +398,7 @@ class Film:
         """8-bit sRGB (h, w, 3) of the film: render_image's denoise plus
         argent-post's develop, on the device."""
         g = grade if grade is not None else N.ArgentGrade(0.0, N.TM_AGX, N.AGX_PUNCHY, 1.0)
-        out = np.zeros((self.height, self.width, 3), np.uint8)
+        out = _results.array((self.height, self.width, 3), np.uint8)
         self.ctx.check(self.ctx.lib.argent_film_develop(self.h, ctypes.byref(g), 1 if denoise else 0, _p(out)))
         return out
 
@@ -407,7 +491,7 @@ class Serve:
         """(color, albedo, normal) of a finished request; forgets it."""
         _, w, h = self._scenes[ticket]
         shape = (h, w, 3)
-        c, a, n = np.zeros(shape, np.float32), np.zeros(shape, np.float32), np.zeros(shape, np.float32)
+        c, a, n = (_results.array(shape, np.float32) for _ in range(3))
         fp = ctypes.POINTER(ctypes.c_float)
         self.ctx.check(self.ctx.lib.argent_serve_read(self.h, ticket, _p(c, fp), _p(a, fp), _p(n, fp)))
         del self._scenes[ticket]
@@ -433,7 +517,7 @@ def denoise_atrous(ctx: Context, color, albedo=None, normal=None):
     c = np.ascontiguousarray(color, np.float32)
     a = None if albedo is None else np.ascontiguousarray(albedo, np.float32)
     n = None if normal is None else np.ascontiguousarray(normal, np.float32)
-    out = np.zeros_like(c)
+    out = _results.array(c.shape, np.float32)
     h, w = c.shape[0], c.shape[1]
     ctx.check(ctx.lib.argent_denoise_atrous(ctx.h, w, h, _p(c, fp), _p(a, fp), _p(n, fp), _p(out, fp)))
     return out
@@ -444,7 +528,7 @@ def develop(ctx: Context, rgb, grade=None):
     8-bit sRGB out."""
     g = grade if grade is not None else N.ArgentGrade(0.0, N.TM_AGX, N.AGX_PUNCHY, 1.0)
     c = np.ascontiguousarray(rgb, np.float32)
-    out = np.zeros(c.shape, np.uint8)
+    out = _results.array(c.shape, np.uint8)
     ctx.check(ctx.lib.argent_develop(ctx.h, c.shape[1], c.shape[0], _p(c, ctypes.POINTER(ctypes.c_float)),
                                      ctypes.byref(g), _p(out)))
     return out

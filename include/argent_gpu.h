@@ -229,6 +229,12 @@ const char* argent_last_error(const ArgentCtx* ctx);
 int argent_ctx_sync(ArgentCtx* ctx);
 /* The context's cudaStream_t, as a void pointer. */
 void* argent_ctx_stream(ArgentCtx* ctx);
+/* Page-locked host memory.  Results read into it (films, hits, images) come
+ * straight from the device, without the driver's staging copy; it costs time
+ * to make, so keep and reuse it.  Freed with argent_pinned_free, from any
+ * thread, once no call writes to it. */
+int argent_pinned_alloc(size_t bytes, void** out);
+void argent_pinned_free(void* p);
 
 /*
  * Upload a piece and build its acceleration structure.  Replaces
