@@ -522,19 +522,19 @@ struct BuildTemps {
 };
 
 // Builds the 8-wide BVH of the piece's uploaded triangles on the device
-// (device_build.cuh) and stores nodes, triangle records, depth and bounds
-// in `p`.  `tidx` holds the piece's triangles (x, y, z = vertex indices).
-std::string device_bvh(ArgentCtx* ctx, ArgentPiece* p, const float4* pos, const uint4* tidx, uint32_t nt) {
+// (device_build.cuh) and stores nodes, depth and bounds in `p`, the triangle
+// records in `dt`.  `tidx` holds the piece's triangles (x, y, z = vertex
+// indices), `bounds` the started centroid bounds (k_piece_pack).
+std::string device_bvh(ArgentCtx* ctx, ArgentPiece* p, const float4* pos, const uint4* tidx, uint32_t nt,
+                       uint32_t* bounds, float4* dt) {
   cudaStream_t st = ctx->stream;
   const size_t n = nt, nb = 2 * n - 1;
   BuildTemps tmp{ctx, st};
   const uint32_t tpb = 256;
-  const uint32_t nblk = (uint32_t)std::min<size_t>((n + tpb - 1) / tpb, (size_t)148 * 8);
+  const uint32_t grid = (uint32_t)std::min<size_t>((n + tpb - 1) / tpb, (size_t)148 * 8);
   float* tlo = tmp.get<float>(3 * n);
   float* thi = tmp.get<float>(3 * n);
   float* cen = tmp.get<float>(3 * n);
-  float* blo = tmp.get<float>(3 * (size_t)nblk);
-  float* bhi = tmp.get<float>(3 * (size_t)nblk);
   uint64_t* k0 = tmp.get<uint64_t>(n);
   uint64_t* k1 = tmp.get<uint64_t>(n);
   uint32_t* v0 = tmp.get<uint32_t>(n);
@@ -550,22 +550,17 @@ std::string device_bvh(ArgentCtx* ctx, ArgentPiece* p, const float4* pos, const 
   bn.flag = tmp.get<uint32_t>(nb);
   int2* qa = tmp.get<int2>(n);
   int2* qb = tmp.get<int2>(n);
-  uint32_t* ctr = tmp.get<uint32_t>(4);  // n_out, node_count, tri_count, err
+  // Items per level (64 levels at most), then node_count, tri_count, err.
+  constexpr uint32_t LEVELS = 64, NODES = LEVELS + 1, TRIS = LEVELS + 2, ERR = LEVELS + 3, CTR = LEVELS + 4;
+  uint32_t* ctr = tmp.get<uint32_t>(CTR);
   const size_t max_nodes = std::max<size_t>(1, n - 1);
   uint4* nodes = tmp.get<uint4>(5 * max_nodes);
   if (tmp.err != cudaSuccess) return std::string("device BVH temporaries: ") + cudaGetErrorString(tmp.err);
 
-  void* dt = nullptr;
-  cudaError_t e = device_alloc(ctx, (void**)&dt, n * sizeof(argent::TriRecord));
-  if (e != cudaSuccess) return std::string("device BVH triangles: ") + cudaGetErrorString(e);
-  p->allocs.push_back(dt);
-  p->bytes += n * sizeof(argent::TriRecord);
-
-  db::k_tri_boxes<<<nblk, tpb, 0, st>>>(pos, tidx, nt, tlo, thi, cen, blo, bhi);
-  const uint32_t grid = nblk;
-  db::k_morton<<<grid, tpb, 0, st>>>(cen, nt, blo, bhi, nblk, k0, v0);
+  db::k_tri_boxes<<<grid, tpb, 0, st>>>(pos, tidx, nt, tlo, thi, cen, bounds);
+  db::k_morton<<<grid, tpb, 0, st>>>(cen, nt, bounds, k0, v0);
   size_t sort_bytes = 0;
-  e = cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, k0, k1, v0, v1, (int)n, 0, 63, st);
+  cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, k0, k1, v0, v1, (int)n, 0, 63, st);
   void* sort_tmp = tmp.get<uint8_t>(sort_bytes);
   if (e == cudaSuccess) e = tmp.err;
   if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(sort_tmp, sort_bytes, k0, k1, v0, v1, (int)n, 0, 63, st);
@@ -579,50 +574,54 @@ std::string device_bvh(ArgentCtx* ctx, ArgentPiece* p, const float4* pos, const 
   db::k_boxes_up<<<grid, tpb, 0, st>>>(tlo, thi, v1, nt, bn);
   ++ctx->launches;
 
-  const uint32_t init[4] = {0, 1, 0, 0};
+  uint32_t init[CTR] = {};
+  init[0] = 1;      // level 0: the root
+  init[NODES] = 1;  // wide node 0
   const int2 root = make_int2(0, 0);  // wide node 0 <- binary root (internal 0, or leaf 0 when n = 1)
   e = cudaMemcpyAsync(ctr, init, sizeof(init), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(qa, &root, sizeof(root), cudaMemcpyHostToDevice, st);
-  uint32_t n_in = 1, depth = 0;
   db::Collapse c{};
-  c.n_out = ctr;
-  c.node_count = ctr + 1;
-  c.tri_count = ctr + 2;
-  c.err = ctr + 3;
+  c.node_count = ctr + NODES;
+  c.tri_count = ctr + TRIS;
+  c.err = ctr + ERR;
   c.nodes = nodes;
-  c.tris = (float4*)dt;
+  c.tris = dt;
   c.pos = pos;
   c.tri = tidx;
   c.vals = v1;
-  while (e == cudaSuccess && n_in > 0) {
-    if (++depth > 64) return "device BVH collapse did not finish in 64 levels";
-    c.in = qa;
-    c.n_in = n_in;
-    c.out = qb;
-    e = cudaMemsetAsync(ctr, 0, sizeof(uint32_t), st);
-    if (e != cudaSuccess) break;
-    uint32_t g = (uint32_t)std::min<size_t>((n_in + 127) / 128, (size_t)148 * 16);
-    db::k_collapse<<<g, 128, 0, st>>>(c, bn, nt);
-    ++ctx->launches;
-    e = cudaMemcpyAsync(&n_in, ctr, sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+  // Ten levels per round trip to the host: an eight-wide tree of a million
+  // triangles has seven to ten, and an empty level costs a launch.
+  uint32_t* got = ctx->h_status + 16;
+  float* box = (float*)(got + CTR);
+  uint32_t level = 0;
+  while (e == cudaSuccess) {
+    for (uint32_t i = 0; i < 10 && level < LEVELS; ++i, ++level) {
+      c.in = level & 1 ? qb : qa;
+      c.out = level & 1 ? qa : qb;
+      c.n_in = ctr + level;
+      c.n_out = ctr + level + 1;
+      const uint64_t most = level < 8 ? 1ull << (3 * level) : n;  // items a level can hold
+      db::k_collapse<<<(uint32_t)std::min<uint64_t>((most + 15) / 16, (uint64_t)148 * 8), 128, 0, st>>>(c, bn, nt);
+      ++ctx->launches;
+    }
+    e = cudaMemcpyAsync(got, ctr, CTR * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(box, bn.lo, 3 * sizeof(float), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(box + 3, bn.hi, 3 * sizeof(float), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    std::swap(qa, qb);
+    if (e != cudaSuccess || got[level] == 0) break;
+    if (level == LEVELS) return "device BVH collapse did not finish in 64 levels";
   }
-  uint32_t got[4] = {0, 0, 0, 0};
-  float box[6];
-  if (e == cudaSuccess) e = cudaMemcpyAsync(got, ctr, sizeof(got), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(box, bn.lo, 3 * sizeof(float), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(box + 3, bn.hi, 3 * sizeof(float), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return std::string("device BVH build: ") + cudaGetErrorString(e);
-  if (got[3] & DB_ERR_EXTENT) return "piece extent too large for the node quantisation";
-  if (got[3]) return "device BVH quantisation failed";
-  if (got[2] != nt || got[1] == 0 || got[1] > max_nodes)
+  uint32_t depth = 0;
+  while (depth < LEVELS && got[depth]) ++depth;
+  if (got[ERR] & DB_ERR_EXTENT) return "piece extent too large for the node quantisation";
+  if (got[ERR]) return "device BVH quantisation failed";
+  if (got[TRIS] != nt || got[NODES] == 0 || got[NODES] > max_nodes)
     return "device BVH build lost triangles or nodes";
   if ((uint64_t)depth * 7 + 1 > ARGENT_STACK_SIZE) return "BVH too deep for the traversal stack";
 
   void* dn = nullptr;
-  const size_t node_bytes = (size_t)got[1] * sizeof(argent::WideNode);
+  const size_t node_bytes = (size_t)got[NODES] * sizeof(argent::WideNode);
   e = device_alloc(ctx, (void**)&dn, node_bytes);
   if (e != cudaSuccess) return std::string("device BVH nodes: ") + cudaGetErrorString(e);
   p->allocs.push_back(dn);
@@ -631,7 +630,7 @@ std::string device_bvh(ArgentCtx* ctx, ArgentPiece* p, const float4* pos, const 
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return std::string("device BVH nodes: ") + cudaGetErrorString(e);
   p->dev.nodes = (const uint4*)dn;
-  p->dev.tris = (const float4*)dt;
+  p->dev.tris = dt;
   p->depth = depth;
   for (int a = 0; a < 3; ++a) {
     p->lo[a] = box[a];
@@ -653,55 +652,77 @@ int argent_piece_upload_device_bvh(ArgentCtx* ctx, const float* positions, uint3
   // An empty piece has nothing to build: the host path makes the same empty piece.
   if (nt == 0) return argent_piece_upload(ctx, positions, nv, normals, tris, nt, tri_material, cavity, out);
   if (nt >= (1u << 27)) return set_error(ctx, ARGENT_E_INVALID, "device BVH build takes fewer than 2^27 triangles");
-  for (uint64_t i = 0; i < 3ull * nt; ++i)
-    if (tris[i] >= nv) return set_error(ctx, ARGENT_E_INVALID, "triangle index out of range");
-  for (uint64_t i = 0; i < 3ull * nv; ++i)
-    if (!std::isfinite(positions[i])) return set_error(ctx, ARGENT_E_INVALID, "non-finite vertex position");
+  if (nv == 0) return set_error(ctx, ARGENT_E_INVALID, "triangle index out of range");
   ARGENT_CK(ctx, cudaSetDevice(ctx->device));
   ArgentPiece* p = new ArgentPiece();
   p->ctx = ctx;
   p->nv = nv;
   p->nt = nt;
-  std::vector<float4> pos4(nv), nrm4;
-  for (uint32_t i = 0; i < nv; ++i) pos4[i] = make_float4(positions[3 * i], positions[3 * i + 1], positions[3 * i + 2], 0);
-  if (normals) {
-    nrm4.resize(nv);
-    for (uint32_t i = 0; i < nv; ++i) nrm4[i] = make_float4(normals[3 * i], normals[3 * i + 1], normals[3 * i + 2], 0);
-  }
-  std::vector<uint4> tidx(nt);
-  for (uint32_t i = 0; i < nt; ++i)
-    tidx[i] = make_uint4(tris[3 * i], tris[3 * i + 1], tris[3 * i + 2], tri_material ? tri_material[i] : 0u);
-  for (uint32_t i = 0; tri_material && i < nt; ++i) p->max_material = std::max<uint32_t>(p->max_material, tri_material[i]);
-  auto up = [&](const void* src, size_t bytes, void** dst) -> cudaError_t {
-    *dst = nullptr;
-    if (bytes == 0) return cudaSuccess;
-    cudaError_t e = device_alloc(ctx, (void**)dst, bytes);
-    if (e != cudaSuccess) return e;
-    p->allocs.push_back(*dst);
-    p->bytes += bytes;
-    return cudaMemcpyAsync(*dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream);
+  cudaStream_t st = ctx->stream;
+  auto fail = [&](int code, const std::string& m) {
+    cudaStreamSynchronize(st);
+    argent_piece_destroy(p);
+    return set_error(ctx, code, m);
   };
-  void *dp = nullptr, *dnr = nullptr, *di = nullptr, *dc = nullptr;
-  cudaError_t e = up(pos4.data(), pos4.size() * sizeof(float4), &dp);
-  if (e == cudaSuccess && normals) e = up(nrm4.data(), nrm4.size() * sizeof(float4), &dnr);
-  if (e == cudaSuccess) e = up(tidx.data(), tidx.size() * sizeof(uint4), &di);
-  if (e == cudaSuccess && cavity) e = up(cavity, (size_t)nv * sizeof(float), &dc);
-  if (e != cudaSuccess) {
-    cudaStreamSynchronize(ctx->stream);
-    std::string m = std::string("piece upload: ") + cudaGetErrorString(e);
-    argent_piece_destroy(p);
-    return set_error(ctx, e == cudaErrorMemoryAllocation ? ARGENT_E_OOM : ARGENT_E_CUDA, m);
+  // The piece's arrays are one allocation (but for the nodes, whose number
+  // the build finds), each on a 256-byte boundary.
+  size_t bytes = 0;
+  auto place = [&](size_t n) {
+    size_t at = bytes;
+    bytes += (n + 255) / 256 * 256;
+    return at;
+  };
+  const size_t o_pos = place((size_t)nv * sizeof(float4)), o_nrm = place(normals ? (size_t)nv * sizeof(float4) : 0),
+               o_idx = place((size_t)nt * sizeof(uint4)), o_cav = place(cavity ? (size_t)nv * sizeof(float) : 0),
+               o_tri = place((size_t)nt * sizeof(argent::TriRecord));
+  uint8_t* base = nullptr;
+  cudaError_t e = device_alloc(ctx, (void**)&base, bytes);
+  if (e != cudaSuccess)
+    return fail(e == cudaErrorMemoryAllocation ? ARGENT_E_OOM : ARGENT_E_CUDA,
+                std::string("piece upload: ") + cudaGetErrorString(e));
+  p->allocs.push_back(base);
+  p->bytes += bytes;
+  float4* pos4 = (float4*)(base + o_pos);
+  float4* nrm4 = normals ? (float4*)(base + o_nrm) : nullptr;
+  uint4* tidx = (uint4*)(base + o_idx);
+  {
+    // The caller's arrays as they are; the device lays them out and checks
+    // them (on the host that took a pass over every vertex and triangle).
+    BuildTemps tmp{ctx, st};
+    float* rp = tmp.get<float>(3 * (size_t)nv);
+    float* rn = normals ? tmp.get<float>(3 * (size_t)nv) : nullptr;
+    uint32_t* rt = tmp.get<uint32_t>(3 * (size_t)nt);
+    uint16_t* rm = tri_material ? tmp.get<uint16_t>(nt) : nullptr;
+    uint32_t* info = tmp.get<uint32_t>(8);
+    if (tmp.err != cudaSuccess)
+      return fail(tmp.err == cudaErrorMemoryAllocation ? ARGENT_E_OOM : ARGENT_E_CUDA,
+                  std::string("piece upload: ") + cudaGetErrorString(tmp.err));
+    auto up = [&](void* d, const void* src, size_t n) {
+      if (e == cudaSuccess) e = cudaMemcpyAsync(d, src, n, cudaMemcpyHostToDevice, st);
+    };
+    up(rp, positions, 3 * (size_t)nv * sizeof(float));
+    if (rn) up(rn, normals, 3 * (size_t)nv * sizeof(float));
+    up(rt, tris, 3 * (size_t)nt * sizeof(uint32_t));
+    if (rm) up(rm, tri_material, (size_t)nt * sizeof(uint16_t));
+    if (cavity) up(base + o_cav, cavity, (size_t)nv * sizeof(float));
+    if (e == cudaSuccess) e = cudaMemsetAsync(info, 0, 2 * sizeof(uint32_t), st);
+    if (e == cudaSuccess) {
+      db::k_piece_pack<<<(uint32_t)ctx->num_sms * 8, 256, 0, st>>>(rp, rn, rt, rm, nv, nt, pos4, nrm4, tidx, info);
+      ++ctx->launches;
+      e = cudaMemcpyAsync(ctx->h_status + 4, info, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return fail(ARGENT_E_CUDA, std::string("piece upload: ") + cudaGetErrorString(e));
+    if (ctx->h_status[4] & DB_BAD_INDEX) return fail(ARGENT_E_INVALID, "triangle index out of range");
+    if (ctx->h_status[4] & DB_BAD_POSITION) return fail(ARGENT_E_INVALID, "non-finite vertex position");
+    p->max_material = ctx->h_status[5];
+    std::string err = device_bvh(ctx, p, pos4, tidx, nt, info + 2, (float4*)(base + o_tri));
+    if (!err.empty()) return fail(ARGENT_E_INVALID, err);
   }
-  std::string err = device_bvh(ctx, p, (const float4*)dp, (const uint4*)di, nt);
-  cudaStreamSynchronize(ctx->stream);
-  if (!err.empty()) {
-    argent_piece_destroy(p);
-    return set_error(ctx, ARGENT_E_INVALID, err);
-  }
-  p->dev.pos = (const float4*)dp;
-  p->dev.nrm = (const float4*)dnr;
-  p->dev.tri_idx = (const uint4*)di;
-  p->dev.cavity = (const float*)dc;
+  p->dev.pos = pos4;
+  p->dev.nrm = nrm4;
+  p->dev.tri_idx = tidx;
+  p->dev.cavity = cavity ? (const float*)(base + o_cav) : nullptr;
   p->dev.num_tris = nt;
   *out = p;
   return ARGENT_OK;

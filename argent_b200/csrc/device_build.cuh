@@ -33,10 +33,54 @@ struct Bin {
   uint32_t* flag;
 };
 
-// Per triangle: box and centroid; block-reduced centroid bounds.  Launched
-// with 256 threads per block.
+// Floats as unsigned words of the same order, for atomicMin and atomicMax.
+__device__ __forceinline__ uint32_t ordered(float f) {
+  uint32_t u = __float_as_uint(f);
+  return u & 0x80000000u ? ~u : u | 0x80000000u;
+}
+__device__ __forceinline__ float unordered(uint32_t u) {
+  return __uint_as_float(u & 0x80000000u ? u & 0x7fffffffu : ~u);
+}
+
+#define DB_BAD_INDEX 1u
+#define DB_BAD_POSITION 2u
+
+// A piece's arrays as the kernels read them, from the caller's: vertices and
+// normals in 16 bytes, triangles with their material slot.  info[0] collects
+// what is wrong with them, info[1] the highest material slot; info[2..7] start
+// the centroid bounds.
+__global__ void __launch_bounds__(256) k_piece_pack(const float* __restrict__ pos, const float* __restrict__ nrm,
+                                                    const uint32_t* __restrict__ tri,
+                                                    const uint16_t* __restrict__ mat, uint32_t nv, uint32_t nt,
+                                                    float4* pos4, float4* nrm4, uint4* tidx, uint32_t* info) {
+  const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  uint32_t bad = 0, top = 0;
+  if (t0 < 6) info[2 + t0] = t0 < 3 ? 0xffffffffu : 0u;
+  for (uint32_t i = t0; i < nv; i += stride) {
+    const float x = pos[3 * (size_t)i], y = pos[3 * (size_t)i + 1], z = pos[3 * (size_t)i + 2];
+    if (!(isfinite(x) && isfinite(y) && isfinite(z))) bad |= DB_BAD_POSITION;
+    pos4[i] = make_float4(x, y, z, 0.0f);
+    if (nrm) nrm4[i] = make_float4(nrm[3 * (size_t)i], nrm[3 * (size_t)i + 1], nrm[3 * (size_t)i + 2], 0.0f);
+  }
+  for (uint32_t i = t0; i < nt; i += stride) {
+    const uint32_t a = tri[3 * (size_t)i], b = tri[3 * (size_t)i + 1], c = tri[3 * (size_t)i + 2];
+    const uint32_t m = mat ? mat[i] : 0u;
+    if (a >= nv || b >= nv || c >= nv) bad |= DB_BAD_INDEX;
+    top = max(top, m);
+    tidx[i] = make_uint4(a, b, c, m);
+  }
+  bad = __reduce_or_sync(0xffffffffu, bad);
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((threadIdx.x & 31) == 0) {
+    if (bad) atomicOr(info, bad);
+    if (top) atomicMax(info + 1, top);
+  }
+}
+
+// Per triangle: box and centroid; the centroid bounds (ordered words, three
+// minima and three maxima).  Launched with 256 threads per block.
 __global__ void __launch_bounds__(256) k_tri_boxes(const float4* pos, const uint4* tri, uint32_t n, float* tlo,
-                                                   float* thi, float* cen, float* blk_lo, float* blk_hi) {
+                                                   float* thi, float* cen, uint32_t* bounds) {
   __shared__ float slo[3][256], shi[3][256];
   float clo[3] = {INFINITY, INFINITY, INFINITY}, chi[3] = {-INFINITY, -INFINITY, -INFINITY};
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
@@ -66,11 +110,10 @@ __global__ void __launch_bounds__(256) k_tri_boxes(const float4* pos, const uint
       }
     __syncthreads();
   }
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 3; ++k) {
-      blk_lo[3 * blockIdx.x + k] = slo[k][0];
-      blk_hi[3 * blockIdx.x + k] = shi[k][0];
-    }
+  if (threadIdx.x < 3) {
+    atomicMin(bounds + threadIdx.x, ordered(slo[threadIdx.x][0]));
+    atomicMax(bounds + 3 + threadIdx.x, ordered(shi[threadIdx.x][0]));
+  }
 }
 
 __device__ __forceinline__ uint64_t spread21(uint32_t v) {
@@ -83,16 +126,15 @@ __device__ __forceinline__ uint64_t spread21(uint32_t v) {
   return x;
 }
 
-// 63-bit Morton code of each centroid within the centroid bounds (every
-// thread reduces the few per-block partials itself).
-__global__ void k_morton(const float* cen, uint32_t n, const float* blk_lo, const float* blk_hi, uint32_t nblk,
-                         uint64_t* keys, uint32_t* vals) {
-  float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-  for (uint32_t b = 0; b < nblk; ++b)
-    for (int k = 0; k < 3; ++k) {
-      lo[k] = fminf(lo[k], blk_lo[3 * b + k]);
-      hi[k] = fmaxf(hi[k], blk_hi[3 * b + k]);
-    }
+// 63-bit Morton code of each centroid within the centroid bounds.  (With
+// per-block partial bounds that every thread reduced for itself, this took
+// 302 us for 500k triangles, a fifth of the build's kernels.)
+__global__ void k_morton(const float* cen, uint32_t n, const uint32_t* bounds, uint64_t* keys, uint32_t* vals) {
+  float lo[3], hi[3];
+  for (int k = 0; k < 3; ++k) {
+    lo[k] = unordered(bounds[k]);
+    hi[k] = unordered(bounds[3 + k]);
+  }
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     uint32_t q[3];
     for (int k = 0; k < 3; ++k) {
@@ -200,7 +242,7 @@ __device__ bool quant_hi(float origin, float v, uint32_t e, uint32_t* out) {
 
 struct Collapse {
   const int2* in;  // (wide node, binary node) of this level
-  uint32_t n_in;
+  const uint32_t* n_in;
   int2* out;
   uint32_t* n_out;
   uint32_t* node_count;
@@ -224,50 +266,103 @@ __device__ __forceinline__ float half_area(const Bin& bn, int32_t b) {
 
 // One level of the collapse: each item fills one wide node from the binary
 // subtree below it (host/bvh_build.cpp Collapser::fill) and queues its
-// interior children for the next level.
-__global__ void k_collapse(Collapse c, Bin bn, uint32_t n) {
-  for (uint32_t it = blockIdx.x * blockDim.x + threadIdx.x; it < c.n_in; it += gridDim.x * blockDim.x) {
-    int2 item = c.in[it];
-    int32_t kids[8];
+// interior children for the next level.  Eight lanes per item, a lane per
+// child: a level is as slow as one item's chain of loads, and a lone thread
+// walked the children's areas, boxes and double-precision quantisation one
+// after the other (60 to 120 us a level at any number of items, eight levels
+// for 500k triangles; now about a tenth).  The level's length is read on the
+// device, so levels follow each other without a copy to the host.
+__global__ void __launch_bounds__(128) k_collapse(Collapse c, Bin bn, uint32_t n) {
+  const unsigned full = 0xffffffffu;
+  const unsigned lane = threadIdx.x & 31u, me = lane & 7u, g0 = lane & 24u;
+  const uint32_t n_in = *c.n_in;
+  const uint32_t warps = gridDim.x * (blockDim.x >> 5), warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  for (uint32_t base = warp * 4; base < n_in; base += warps * 4) {
+    const uint32_t it = base + (lane >> 3);
+    const bool on = it < n_in;
+    int2 item = on ? c.in[it] : make_int2(0, 0);
+    // This lane's child: its binary node, whether it may be opened, and its
+    // half area if so (-1 otherwise).
+    int32_t kid = -1;
+    float area = -1.0f;
     int nk = 0;
-    if (leafish(bn, n, item.y)) {
-      kids[nk++] = item.y;
-    } else {
-      kids[nk++] = bn.left[item.y];
-      kids[nk++] = bn.right[item.y];
-    }
-    while (nk < 8) {
-      int best = -1;
-      float best_a = -1.0f;
-      for (int i = 0; i < nk; ++i)
-        if (!leafish(bn, n, kids[i])) {
-          float a = half_area(bn, kids[i]);
-          if (a > best_a) {
-            best = i;
-            best_a = a;
-          }
-        }
-      if (best < 0) break;
-      int32_t open = kids[best];
-      for (int i = nk; i > best + 1; --i) kids[i] = kids[i - 1];
-      kids[best] = bn.left[open];
-      kids[best + 1] = bn.right[open];
-      ++nk;
-    }
-    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (int i = 0; i < nk; ++i)
-      for (int a = 0; a < 3; ++a) {
-        lo[a] = fminf(lo[a], bn.lo[3 * (size_t)kids[i] + a]);
-        hi[a] = fmaxf(hi[a], bn.hi[3 * (size_t)kids[i] + a]);
+    auto take = [&](int32_t b) {
+      kid = b;
+      area = leafish(bn, n, b) ? -1.0f : half_area(bn, b);
+    };
+    if (on) {
+      if (leafish(bn, n, item.y)) {
+        nk = 1;
+        if (me == 0) take(item.y);
+      } else {
+        nk = 2;
+        if (me == 0) take(bn.left[item.y]);
+        if (me == 1) take(bn.right[item.y]);
       }
-    uint32_t e[3];
+    }
+    for (;;) {
+      // The first of the largest areas among the children that can be opened.
+      float best_a = area;
+      unsigned best = me;
+#pragma unroll
+      for (int i = 1; i < 8; i <<= 1) {
+        const float oa = __shfl_xor_sync(full, best_a, i);
+        const unsigned ob = __shfl_xor_sync(full, best, i);
+        if (oa > best_a || (oa == best_a && ob < best)) {
+          best_a = oa;
+          best = ob;
+        }
+      }
+      const bool open = on && nk < 8 && best_a > -1.0f;
+      if (__ballot_sync(full, open) == 0) break;
+      const int32_t opened = __shfl_sync(full, kid, (int)(g0 + best));
+      const int32_t up_kid = __shfl_up_sync(full, kid, 1);
+      const float up_area = __shfl_up_sync(full, area, 1);
+      if (open) {
+        if (me == best) {
+          take(bn.left[opened]);
+        } else if (me == best + 1) {
+          take(bn.right[opened]);
+        } else if (me > best + 1) {
+          kid = up_kid;
+          area = up_area;
+        }
+        ++nk;
+      }
+    }
+    const bool have = on && (int)me < nk;
+    float klo[3] = {INFINITY, INFINITY, INFINITY}, khi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    uint32_t first = 0, last = 0;
+    bool leaf = false;
+    if (have) {
+      leaf = leafish(bn, n, kid);
+      first = bn.first[kid];
+      last = bn.last[kid];
+      for (int a = 0; a < 3; ++a) {
+        klo[a] = bn.lo[3 * (size_t)kid + a];
+        khi[a] = bn.hi[3 * (size_t)kid + a];
+      }
+    }
+    float lo[3], hi[3];
     for (int a = 0; a < 3; ++a) {
-      float ext = hi[a] - lo[a];
+      lo[a] = klo[a];
+      hi[a] = khi[a];
+#pragma unroll
+      for (int i = 1; i < 8; i <<= 1) {
+        lo[a] = fminf(lo[a], __shfl_xor_sync(full, lo[a], i));
+        hi[a] = fmaxf(hi[a], __shfl_xor_sync(full, hi[a], i));
+      }
+    }
+    // The axes' exponents: a lane per axis.
+    uint32_t ex = 0;
+    if (on && me < 3) {
+      const float l = me == 0 ? lo[0] : me == 1 ? lo[1] : lo[2], h = me == 0 ? hi[0] : me == 1 ? hi[1] : hi[2];
+      float ext = h - l;
       int ee = -120;
       if (ext > 0.0f) {
-        int ex;
-        frexp((double)ext / 255.0, &ex);
-        ee = ex;
+        int x;
+        frexp((double)ext / 255.0, &x);
+        ee = x;
       }
       ee = max(ee, -120);
       if (ee > 60) {
@@ -275,62 +370,89 @@ __global__ void k_collapse(Collapse c, Bin bn, uint32_t n) {
         ee = 60;
       }
       uint32_t qh;
-      while (ee <= 60 && !quant_hi(lo[a], hi[a], (uint32_t)(ee + 127), &qh)) ++ee;
+      while (ee <= 60 && !quant_hi(l, h, (uint32_t)(ee + 127), &qh)) ++ee;
       if (ee > 60) {
         atomicOr(c.err, DB_ERR_QUANT);
         ee = 60;
       }
-      e[a] = (uint32_t)(ee + 127);
+      ex = (uint32_t)(ee + 127);
     }
-    uint32_t n_int = 0, n_tri = 0;
-    for (int i = 0; i < nk; ++i) {
-      if (leafish(bn, n, kids[i]))
-        n_tri += bn.last[kids[i]] - bn.first[kids[i]] + 1;
-      else
-        ++n_int;
+    uint32_t e[3];
+    for (int a = 0; a < 3; ++a) e[a] = __shfl_sync(full, ex, (int)g0 + a);
+    // Bases of the item's interior children and triangles.
+    const unsigned im = (__ballot_sync(full, have && !leaf) >> g0) & 0xffu;
+    const unsigned pm = (__ballot_sync(full, have) >> g0) & 0xffu;
+    const uint32_t cnt = have && leaf ? last - first + 1u : 0u;
+    uint32_t toff = cnt;  // inclusive sum over the lanes before and this one
+#pragma unroll
+    for (int i = 1; i < 8; i <<= 1) {
+      const uint32_t x = __shfl_up_sync(full, toff, i);
+      if ((int)me >= i) toff += x;
     }
-    uint32_t child_base = n_int ? atomicAdd(c.node_count, n_int) : 0u;
-    uint32_t tri_base = n_tri ? atomicAdd(c.tri_count, n_tri) : 0u;
-    uint32_t imask = 0, present = 0, counts = 0;
-    uint32_t q[6][2] = {{0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}, {0, 0}};  // qlo x,y,z then qhi x,y,z
-    uint32_t slot = 0, toff = 0;
-    for (int i = 0; i < nk; ++i) {
-      int32_t k = kids[i];
-      present |= 1u << i;
-      for (int a = 0; a < 3; ++a) {
-        uint32_t ql = quant_lo(lo[a], bn.lo[3 * (size_t)k + a], e[a]);
-        uint32_t qh = 255;
-        if (!quant_hi(lo[a], bn.hi[3 * (size_t)k + a], e[a], &qh)) atomicOr(c.err, DB_ERR_QUANT);
-        q[a][i >> 2] |= ql << (8 * (i & 3));
-        q[3 + a][i >> 2] |= qh << (8 * (i & 3));
+    const uint32_t n_tri = __shfl_sync(full, toff, (int)g0 + 7), n_int = (uint32_t)__popc(im);
+    toff -= cnt;
+    uint32_t child_base = 0, tri_base = 0, out_base = 0;
+    if (on && me == 0) {
+      if (n_int) {
+        child_base = atomicAdd(c.node_count, n_int);
+        out_base = atomicAdd(c.n_out, n_int);
       }
-      if (leafish(bn, n, k)) {
-        uint32_t f = bn.first[k], l = bn.last[k];
-        counts |= (l - f) << (4 * i);
-        for (uint32_t s = f; s <= l; ++s) {
+      if (n_tri) tri_base = atomicAdd(c.tri_count, n_tri);
+    }
+    child_base = __shfl_sync(full, child_base, (int)g0);
+    tri_base = __shfl_sync(full, tri_base, (int)g0);
+    out_base = __shfl_sync(full, out_base, (int)g0);
+    uint32_t q[6] = {0, 0, 0, 0, 0, 0};  // this child's planes: lo x, y, z then hi x, y, z
+    if (have) {
+      for (int a = 0; a < 3; ++a) {
+        q[a] = quant_lo(lo[a], klo[a], e[a]);
+        q[3 + a] = 255;
+        if (!quant_hi(lo[a], khi[a], e[a], &q[3 + a])) atomicOr(c.err, DB_ERR_QUANT);
+      }
+      if (leaf) {
+        for (uint32_t s = first; s <= last; ++s) {
           uint32_t t = c.vals[s];
           uint4 ti = c.tri[t];
           float4 a = c.pos[ti.x], b = c.pos[ti.y], d = c.pos[ti.z];
-          size_t o = 3 * (size_t)(tri_base + toff);
+          size_t o = 3 * (size_t)(tri_base + toff + (s - first));
           c.tris[o] = make_float4(a.x, a.y, a.z, __uint_as_float(t));
           c.tris[o + 1] = make_float4(__fsub_rn(b.x, a.x), __fsub_rn(b.y, a.y), __fsub_rn(b.z, a.z), 0.0f);
           c.tris[o + 2] = make_float4(__fsub_rn(d.x, a.x), __fsub_rn(d.y, a.y), __fsub_rn(d.z, a.z), 0.0f);
-          ++toff;
         }
       } else {
-        imask |= 1u << i;
-        uint32_t o = atomicAdd(c.n_out, 1u);
-        c.out[o] = make_int2((int)(child_base + slot), k);
-        ++slot;
+        const uint32_t slot = (uint32_t)__popc(im & ((1u << me) - 1u));
+        c.out[out_base + slot] = make_int2((int)(child_base + slot), kid);
       }
     }
-    uint4* w = c.nodes + 5 * (size_t)item.x;
-    w[0] = make_uint4(__float_as_uint(lo[0]), __float_as_uint(lo[1]), __float_as_uint(lo[2]),
-                      e[0] | (e[1] << 8) | (e[2] << 16) | (imask << 24));
-    w[1] = make_uint4(child_base, tri_base, counts, present);
-    w[2] = make_uint4(q[0][0], q[0][1], q[1][0], q[1][1]);
-    w[3] = make_uint4(q[2][0], q[2][1], q[3][0], q[3][1]);
-    w[4] = make_uint4(q[4][0], q[4][1], q[5][0], q[5][1]);
+    // Packed words: each lane's byte (and leaf count) into its place.
+    const uint32_t sh = 8 * (me & 3);
+    uint32_t counts = cnt ? (cnt - 1u) << (4 * me) : 0u;
+#pragma unroll
+    for (int i = 1; i < 8; i <<= 1) counts |= __shfl_xor_sync(full, counts, i);
+    uint32_t pw[6][2];
+#pragma unroll
+    for (int a = 0; a < 6; ++a) {
+      uint32_t x = q[a] << sh;  // halves of the group: lanes 0-3 and 4-7
+      x |= __shfl_xor_sync(full, x, 1);
+      x |= __shfl_xor_sync(full, x, 2);
+      pw[a][0] = __shfl_sync(full, x, (int)g0);
+      pw[a][1] = __shfl_sync(full, x, (int)g0 + 4);
+    }
+    if (on && me < 5) {
+      uint4 w;
+      if (me == 0)
+        w = make_uint4(__float_as_uint(lo[0]), __float_as_uint(lo[1]), __float_as_uint(lo[2]),
+                       e[0] | (e[1] << 8) | (e[2] << 16) | (im << 24));
+      else if (me == 1)
+        w = make_uint4(child_base, tri_base, counts, pm);
+      else if (me == 2)
+        w = make_uint4(pw[0][0], pw[0][1], pw[1][0], pw[1][1]);
+      else if (me == 3)
+        w = make_uint4(pw[2][0], pw[2][1], pw[3][0], pw[3][1]);
+      else
+        w = make_uint4(pw[4][0], pw[4][1], pw[5][0], pw[5][1]);
+      c.nodes[5 * (size_t)item.x + me] = w;
+    }
   }
 }
 
