@@ -53,34 +53,111 @@ int set_error(const ArgentCtx* ctx, int code, const std::string& msg) {
 
 // ------------------------------------------------------------------ kernels
 
-__global__ void k_trace_closest(DevPiece pc, const ArgentRay* __restrict__ rays, uint64_t n, ArgentHit* hits,
-                                uint32_t* status) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    const float4* rp = reinterpret_cast<const float4*>(rays + i);
-    float4 a = __ldg(rp), b = __ldg(rp + 1);
-    TraceHit h = trace_closest(pc, V3{a.x, a.y, a.z}, V3{b.x, b.y, b.z}, a.w, status);
-    ArgentHit o;
-    if (h.prim == ARGENT_NO_HIT_U) {
-      o.t = 0.0f;
-      o.u = 0.0f;
-      o.v = 0.0f;
-    } else {
-      o.t = h.t;
-      o.u = h.u;
-      o.v = h.v;
+// The whole queue of a trace call on persistent lanes, as in k_intersect and
+// k_shadow: a lane takes a new ray as soon as a warp has ARGENT_REFILL idle
+// ones, and each step the lanes at a leaf or the lanes at a node visit,
+// whichever are more.  With a thread per ray a warp ran until its slowest ray
+// ended: a million rays from round and off a 2.1M-triangle piece took 955 us,
+// now 790-840 (ncu, cold), the patina mask's 6 M hemisphere rays on 250k
+// triangles 2100, now 1193.  `work` is zero at the start.
+template <class SRC>
+__device__ __forceinline__ void trace_closest_queue(const DevPiece& pc, uint32_t count, uint32_t* work, SRC src,
+                                                    uint32_t* status) {
+  uint2 arr[ARGENT_STACK_SIZE];
+  LocalStack<uint2> stack{arr};
+  ClosestTrav s;
+  uint32_t idx = 0;
+  bool active = false, running = false, first = true, more = true;
+  for (;;) {
+    const uint32_t j = lane_refill(!active, &first, &more, count, work);
+    if (j != ~0u) {
+      idx = j;
+      V3 o, d;
+      float t_max;
+      src.ray(j, &o, &d, &t_max);
+      running = closest_begin(pc, s, o, d, t_max);
+      active = true;
     }
-    o.prim = h.prim;
-    reinterpret_cast<float4*>(hits)[i] = make_float4(o.t, o.u, o.v, __uint_as_float(o.prim));
+    if (__ballot_sync(0xffffffffu, active) == 0 && !more) break;
+    if (active && running) running = closest_next(s, stack);
+    const bool run = active && running, at_leaf = run && trav_at_leaf(s.ref), at_node = run && !trav_at_leaf(s.ref);
+    const bool leaves =
+        __popc(__ballot_sync(0xffffffffu, at_leaf)) >= __popc(__ballot_sync(0xffffffffu, at_node));
+    if (leaves ? at_leaf : at_node) running = closest_visit(pc, s, stack, status);
+    if (active && !running) {
+      count_visits(0, s.n_nodes, s.n_tris);
+      src.done(idx, s.best);
+      active = false;
+    }
   }
 }
 
-__global__ void k_trace_any(DevPiece pc, const ArgentRay* __restrict__ rays, uint64_t n, uint8_t* occ,
-                            uint32_t* status) {
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    const float4* rp = reinterpret_cast<const float4*>(rays + i);
-    float4 a = __ldg(rp), b = __ldg(rp + 1);
-    occ[i] = trace_any(pc, V3{a.x, a.y, a.z}, V3{b.x, b.y, b.z}, a.w, status) ? 1 : 0;
+template <class SRC>
+__device__ __forceinline__ void trace_any_queue(const DevPiece& pc, uint32_t count, uint32_t* work, SRC src,
+                                                uint32_t* status) {
+  uint32_t arr[ARGENT_STACK_SIZE];
+  LocalStack<uint32_t> stack{arr};
+  AnyTrav s;
+  uint32_t idx = 0;
+  int state = ARGENT_ANY_CLEAR;
+  bool active = false, first = true, more = true;
+  for (;;) {
+    const uint32_t j = lane_refill(!active, &first, &more, count, work);
+    if (j != ~0u) {
+      idx = j;
+      V3 o, d;
+      float t_max;
+      active = src.ray(j, &o, &d, &t_max);
+      if (active) state = any_begin(pc, s, stack, o, d, t_max);
+    }
+    if (__ballot_sync(0xffffffffu, active) == 0 && !more) break;
+    if (active && state == ARGENT_ANY_RUNNING && !any_next(s, stack)) state = ARGENT_ANY_CLEAR;
+    const bool run = active && state == ARGENT_ANY_RUNNING, at_leaf = run && trav_at_leaf(s.ref),
+               at_node = run && !trav_at_leaf(s.ref);
+    const bool leaves =
+        __popc(__ballot_sync(0xffffffffu, at_leaf)) >= __popc(__ballot_sync(0xffffffffu, at_node));
+    if (leaves ? at_leaf : at_node) state = any_visit(pc, s, stack, status);
+    if (active && state != ARGENT_ANY_RUNNING) {
+      count_visits(3, s.n_nodes, s.n_tris);
+      src.done(idx, state == ARGENT_ANY_HIT);
+      active = false;
+    }
   }
+}
+
+struct RaySource {
+  const ArgentRay* __restrict__ rays;
+  __device__ __forceinline__ bool ray(uint32_t j, V3* o, V3* d, float* t_max) const {
+    const float4* rp = reinterpret_cast<const float4*>(rays + j);
+    const float4 a = __ldg(rp), b = __ldg(rp + 1);
+    *o = V3{a.x, a.y, a.z};
+    *d = V3{b.x, b.y, b.z};
+    *t_max = a.w;
+    return true;
+  }
+};
+struct ClosestRays : RaySource {
+  ArgentHit* hits;
+  __device__ __forceinline__ void done(uint32_t j, const TraceHit& h) const {
+    const bool miss = h.prim == ARGENT_NO_HIT_U;
+    reinterpret_cast<float4*>(hits)[j] =
+        make_float4(miss ? 0.0f : h.t, miss ? 0.0f : h.u, miss ? 0.0f : h.v, __uint_as_float(h.prim));
+  }
+};
+struct AnyRays : RaySource {
+  uint8_t* occ;
+  __device__ __forceinline__ void done(uint32_t j, bool hit) const { occ[j] = hit ? 1 : 0; }
+};
+
+__global__ void __launch_bounds__(128, ARGENT_TRAV_BLOCKS)
+    k_trace_closest(DevPiece pc, const ArgentRay* rays, uint32_t n, ArgentHit* hits, uint32_t* work,
+                    uint32_t* status) {
+  trace_closest_queue(pc, n, work, ClosestRays{{rays}, hits}, status);
+}
+
+__global__ void __launch_bounds__(128, ARGENT_TRAV_BLOCKS)
+    k_trace_any(DevPiece pc, const ArgentRay* rays, uint32_t n, uint8_t* occ, uint32_t* work, uint32_t* status) {
+  trace_any_queue(pc, n, work, AnyRays{{rays}, occ}, status);
 }
 
 // The same for calls too small to fill the device with a thread per ray:
@@ -146,22 +223,24 @@ __global__ void k_tri_records(float4* tris, const uint4* __restrict__ tri_idx, c
 
 // ------------------------------------------------------------------ cavity ambient occlusion
 
-// cavity.rs:96-135, one thread per (vertex, sample): the ray from the
-// vertex nudged eps along its normal, direction from a cosine-weighted
-// stratified hemisphere rotated by a vertex hash, tested for any hit within
-// `distance` (the Occluder of scene.rs:40-44).  Consecutive threads are
-// samples of one vertex, so a warp's rays share an origin.  glam's
-// normalize_or_zero and any_orthonormal_pair (Duff et al. 2017, sign =
-// signum(z)) are restated in glam's scalar operation order.
-__global__ void __launch_bounds__(128) k_cavity_ao(DevPiece pc, const float* __restrict__ normals, uint32_t nv,
-                                                   uint32_t n, float distance, float eps, uint32_t* counts,
-                                                   uint32_t* status) {
-  uint64_t total = (uint64_t)nv * n;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t v = (uint32_t)(i / n), k = (uint32_t)(i % n);
+// cavity.rs:96-135, one ray per (vertex, sample): from the vertex nudged eps
+// along its normal, in a direction of a cosine-weighted stratified hemisphere
+// rotated by a vertex hash, tested for any hit within `distance` (the Occluder
+// of scene.rs:40-44).  Consecutive rays are samples of one vertex, so a warp's
+// rays share an origin.  glam's normalize_or_zero and any_orthonormal_pair
+// (Duff et al. 2017, sign = signum(z)) are restated in glam's scalar operation
+// order.
+struct CavityRays {
+  const float4* pos;
+  const float* normals;
+  uint32_t v0, n;  // first vertex of the launch, samples per vertex
+  float distance, eps;
+  uint32_t* counts;
+  __device__ __forceinline__ bool ray(uint32_t j, V3* o, V3* dir, float* t_max) const {
+    const uint32_t v = v0 + j / n, k = j % n;
     float nx = normals[3 * (size_t)v], ny = normals[3 * (size_t)v + 1], nz = normals[3 * (size_t)v + 2];
     float rcp = __fdiv_rn(1.0f, __fsqrt_rn((nx * nx + ny * ny) + nz * nz));
-    if (!(isfinite(rcp) && rcp > 0.0f)) continue;
+    if (!(isfinite(rcp) && rcp > 0.0f)) return false;
     nx *= rcp;
     ny *= rcp;
     nz *= rcp;
@@ -170,8 +249,8 @@ __global__ void __launch_bounds__(128) k_cavity_ao(DevPiece pc, const float* __r
     float bb = nx * ny * a;
     float tx = 1.0f + sign * nx * nx * a, ty = sign * bb, tz = -sign * nx;
     float bx = bb, by = sign + ny * ny * a, bz = -ny;
-    float4 p = __ldg(pc.pos + v);
-    V3 o{p.x + nx * eps, p.y + ny * eps, p.z + nz * eps};
+    float4 p = __ldg(pos + v);
+    *o = V3{p.x + nx * eps, p.y + ny * eps, p.z + nz * eps};
     uint32_t h = hash32(v ^ 0x5bd1e995u);
     float rot = (float)(h >> 8) * (1.0f / 16777216.0f);
     float jit = (float)(hash32(h) >> 8) * (1.0f / 16777216.0f);
@@ -181,9 +260,18 @@ __global__ void __launch_bounds__(128) k_cavity_ao(DevPiece pc, const float* __r
     float r = __fsqrt_rn(u1);
     float phi = 6.28318530717958647692f * u2;
     float c = r * cosf(phi), sn = r * sinf(phi), w = __fsqrt_rn(1.0f - u1);
-    V3 d{(tx * c + bx * sn) + nx * w, (ty * c + by * sn) + ny * w, (tz * c + bz * sn) + nz * w};
-    if (trace_any(pc, o, d, distance, status)) atomicAdd(counts + v, 1u);
+    *dir = V3{(tx * c + bx * sn) + nx * w, (ty * c + by * sn) + ny * w, (tz * c + bz * sn) + nz * w};
+    *t_max = distance;
+    return true;
   }
+  __device__ __forceinline__ void done(uint32_t j, bool hit) const {
+    if (hit) atomicAdd(counts + v0 + j / n, 1u);
+  }
+};
+
+__global__ void __launch_bounds__(128, ARGENT_TRAV_BLOCKS)
+    k_cavity_ao(DevPiece pc, CavityRays rays, uint32_t count, uint32_t* work, uint32_t* status) {
+  trace_any_queue(pc, count, work, rays, status);
 }
 
 __global__ void k_cavity_ao_finish(const uint32_t* counts, uint32_t nv, uint32_t n, float* out) {
@@ -239,6 +327,11 @@ int grid_for(const ArgentCtx* ctx, const void* kernel, int block, uint64_t n) {
   uint64_t g = std::min<uint64_t>(full, (uint64_t)ctx->num_sms * per_sm);
   return (int)std::max<uint64_t>(g, 1);
 }
+
+// Rays of one launch at most, and the status buffer's word that counts the
+// batches they are taken in.
+static constexpr uint64_t TRACE_CHUNK = 1ull << 30;
+static constexpr int TRACE_WORK = 2;
 
 // Blocks of 128 threads for the eight-lanes-per-ray form of a trace of `n`
 // rays (every ray at once, one per warp while warps are free), or 0 when the
@@ -763,13 +856,18 @@ uint64_t argent_piece_device_bytes(const ArgentPiece* p) { return p ? p->bytes :
 
 static void launch_trace_closest(ArgentCtx* ctx, ArgentPiece* piece, const ArgentRay* d_rays, uint64_t n,
                                  ArgentHit* d_hits) {
-  const int few = few_rays_grid(ctx, n);
-  ProfScope ps(ctx, KC_TRACE);
-  if (few)
+  if (const int few = few_rays_grid(ctx, n)) {
+    ProfScope ps(ctx, KC_TRACE);
     k_trace_closest_few<<<few, 128, 0, ctx->stream>>>(piece->dev, d_rays, (uint32_t)n, d_hits, ctx->d_status);
-  else
-    k_trace_closest<<<grid_for(ctx, (const void*)k_trace_closest, 128, n), 128, 0, ctx->stream>>>(
-        piece->dev, d_rays, n, d_hits, ctx->d_status);
+    return;
+  }
+  for (uint64_t at = 0; at < n; at += TRACE_CHUNK) {
+    const uint32_t m = (uint32_t)std::min<uint64_t>(TRACE_CHUNK, n - at);
+    cudaMemsetAsync(ctx->d_status + TRACE_WORK, 0, sizeof(uint32_t), ctx->stream);
+    ProfScope ps(ctx, KC_TRACE);
+    k_trace_closest<<<grid_for(ctx, (const void*)k_trace_closest, 128, m), 128, 0, ctx->stream>>>(
+        piece->dev, d_rays + at, m, d_hits + at, ctx->d_status + TRACE_WORK, ctx->d_status);
+  }
 }
 
 int argent_trace_closest_device(ArgentCtx* ctx, ArgentPiece* piece, const ArgentRay* d_rays, uint64_t n,
@@ -788,14 +886,17 @@ int argent_trace_anyhit_device(ArgentCtx* ctx, ArgentPiece* piece, const ArgentR
   if (!ctx || !piece) return set_error(ctx, ARGENT_E_INVALID, "NULL argument");
   if (n == 0) return ARGENT_OK;
   ARGENT_CK(ctx, cudaSetDevice(ctx->device));
-  const int few = few_rays_grid(ctx, n);
-  {
+  if (const int few = few_rays_grid(ctx, n)) {
     ProfScope ps(ctx, KC_TRACE);
-    if (few)
-      k_trace_any_few<<<few, 128, 0, ctx->stream>>>(piece->dev, d_rays, (uint32_t)n, d_occ, ctx->d_status);
-    else
-      k_trace_any<<<grid_for(ctx, (const void*)k_trace_any, 128, n), 128, 0, ctx->stream>>>(piece->dev, d_rays, n,
-                                                                                          d_occ, ctx->d_status);
+    k_trace_any_few<<<few, 128, 0, ctx->stream>>>(piece->dev, d_rays, (uint32_t)n, d_occ, ctx->d_status);
+  } else {
+    for (uint64_t at = 0; at < n; at += TRACE_CHUNK) {
+      const uint32_t m = (uint32_t)std::min<uint64_t>(TRACE_CHUNK, n - at);
+      ARGENT_CK(ctx, cudaMemsetAsync(ctx->d_status + TRACE_WORK, 0, sizeof(uint32_t), ctx->stream));
+      ProfScope ps(ctx, KC_TRACE);
+      k_trace_any<<<grid_for(ctx, (const void*)k_trace_any, 128, m), 128, 0, ctx->stream>>>(
+          piece->dev, d_rays + at, m, d_occ + at, ctx->d_status + TRACE_WORK, ctx->d_status);
+    }
   }
   ctx->launches++;
   ARGENT_CK(ctx, cudaGetLastError());
@@ -1065,15 +1166,20 @@ int argent_piece_ambient_occlusion(ArgentCtx* ctx, ArgentPiece* piece, const flo
   ARGENT_CK(ctx, scratch_alloc(ctx, (void**)&d_ao, (size_t)nv * sizeof(float)));
   ARGENT_CK(ctx, cudaMemcpyAsync(d_n, normals, 3ull * nv * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
   ARGENT_CK(ctx, cudaMemsetAsync(d_cnt, 0, (size_t)nv * sizeof(uint32_t), ctx->stream));
-  uint64_t total = (uint64_t)nv * samples;
-  int grid = grid_for(ctx, (const void*)k_cavity_ao, 128, total);
-  {
+  // Launches of whole vertices, at most TRACE_CHUNK rays each.
+  const uint32_t step = (uint32_t)std::max<uint64_t>(1, TRACE_CHUNK / samples);
+  uint64_t launches = 1;
+  for (uint64_t v = 0; v < nv; v += step, ++launches) {
+    const uint64_t m = (uint64_t)std::min<uint64_t>(step, nv - v) * samples;
+    CavityRays rays{piece->dev.pos, d_n, (uint32_t)v, samples, distance, eps, d_cnt};
+    ARGENT_CK(ctx, cudaMemsetAsync(ctx->d_status + TRACE_WORK, 0, sizeof(uint32_t), ctx->stream));
     ProfScope ps(ctx, KC_TRACE);
-    k_cavity_ao<<<grid, 128, 0, ctx->stream>>>(piece->dev, d_n, nv, samples, distance, eps, d_cnt, ctx->d_status);
+    k_cavity_ao<<<grid_for(ctx, (const void*)k_cavity_ao, 128, m), 128, 0, ctx->stream>>>(
+        piece->dev, rays, (uint32_t)m, ctx->d_status + TRACE_WORK, ctx->d_status);
   }
   int g2 = (int)std::min<uint64_t>((nv + 255) / 256, (uint64_t)ctx->num_sms * 8);
   k_cavity_ao_finish<<<std::max(g2, 1), 256, 0, ctx->stream>>>(d_cnt, nv, samples, d_ao);
-  ctx->launches += 2;
+  ctx->launches += launches;
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(ao, d_ao, (size_t)nv * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream);

@@ -402,7 +402,7 @@ __device__ __forceinline__ void sort8(uint32_t k[8]) {
 // best at every point, so its box is always entered.
 //
 // The traversal is resumable: closest_begin sets it up and each
-// closest_step visits one node or one leaf, so a kernel can interleave the
+// closest_visit visits one node or one leaf, so a kernel can interleave the
 // steps of rays that start at different times (persistent lanes that take a
 // new ray as soon as theirs finishes).  The stack lives with the caller.
 struct ClosestTrav {
@@ -514,24 +514,6 @@ __device__ __forceinline__ bool closest_visit(const DevPiece& pc, ClosestTrav& s
   return true;
 }
 
-// Visits one node or one leaf; true when the traversal has finished.
-template <class ST>
-__device__ __forceinline__ bool closest_step(const DevPiece& pc, ClosestTrav& s, ST& stack, uint32_t* status) {
-  if (!closest_next(s, stack)) return true;
-  return !closest_visit(pc, s, stack, status);
-}
-
-__device__ __noinline__ TraceHit trace_closest(const DevPiece& pc, V3 o, V3 d, float t_max, uint32_t* status) {
-  ClosestTrav s;
-  uint2 arr[ARGENT_STACK_SIZE];
-  LocalStack<uint2> stack{arr};
-  if (closest_begin(pc, s, o, d, t_max))
-    while (!closest_step(pc, s, stack, status)) {
-    }
-  count_visits(0, s.n_nodes, s.n_tris);
-  return s.best;
-}
-
 // Any hit with t in (1e-7, t_max), bvh.rs:216-247, resumable like the
 // closest-hit traversal.
 struct AnyTrav {
@@ -626,30 +608,13 @@ __device__ __forceinline__ int any_visit(const DevPiece& pc, AnyTrav& s, ST& sta
   return s.sp == 0 ? ARGENT_ANY_CLEAR : ARGENT_ANY_RUNNING;
 }
 
-// Visits one node or one leaf.
-template <class ST>
-__device__ __forceinline__ int any_step(const DevPiece& pc, AnyTrav& s, ST& stack, uint32_t* status) {
-  if (!any_next(s, stack)) return ARGENT_ANY_CLEAR;
-  return any_visit(pc, s, stack, status);
-}
-
-__device__ __noinline__ bool trace_any(const DevPiece& pc, V3 o, V3 d, float t_max, uint32_t* status) {
-  AnyTrav s;
-  uint32_t arr[ARGENT_STACK_SIZE];
-  LocalStack<uint32_t> stack{arr};
-  int r = any_begin(pc, s, stack, o, d, t_max);
-  while (r == ARGENT_ANY_RUNNING) r = any_step(pc, s, stack, status);
-  count_visits(3, s.n_nodes, s.n_tris);
-  return r == ARGENT_ANY_HIT;
-}
-
 // ---------------------------------------------------------------- few rays
 // Traversal by groups of eight lanes, for queues too short to fill the
 // device: a lane per child of a node and per triangle of a leaf, so a ray's
 // chain of steps is several times shorter in time (a lone lane takes the
 // eight slab tests, the sort and the leaf's triangles one after the other).
 // All lanes of a warp call together; the lanes of a group pass the same ray.
-// The hits are those of trace_closest and trace_any: the closest hit is the
+// The hits are those of a thread per ray: the closest hit is the
 // minimum of (t, triangle index) whatever the order of visits, and the boxes
 // are tested by the same arithmetic.
 //

@@ -269,8 +269,8 @@ __device__ __forceinline__ float half_area(const Bin& bn, int32_t b) {
 // interior children for the next level.  Eight lanes per item, a lane per
 // child: a level is as slow as one item's chain of loads, and a lone thread
 // walked the children's areas, boxes and double-precision quantisation one
-// after the other (60 to 120 us a level at any number of items, eight levels
-// for 500k triangles; now about a tenth).  The level's length is read on the
+// after the other (60 to 120 us a level at any number of items, now 24 to 45;
+// 500k triangles have eight levels).  The level's length is read on the
 // device, so levels follow each other without a copy to the host.
 __global__ void __launch_bounds__(128) k_collapse(Collapse c, Bin bn, uint32_t n) {
   const unsigned full = 0xffffffffu;
