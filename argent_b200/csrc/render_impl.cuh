@@ -612,7 +612,7 @@ __global__ void __launch_bounds__(128, ARGENT_TRAV_BLOCKS) k_intersect(WaveArgs 
   }
   ClosestTrav s;
   const DevScene* sc = U ? a.uscene : nullptr;
-  uint32_t slot = 0;
+  uint32_t slot = 0, pf = HIT_MISS;  // pf: the panel or floor hit
   bool active = false, running = false, first = true, more = true;
   for (;;) {
     uint32_t j = lane_refill(!active, &first, &more, count, work);
@@ -620,13 +620,36 @@ __global__ void __launch_bounds__(128, ARGENT_TRAV_BLOCKS) k_intersect(WaveArgs 
       slot = qin[j];
       if (!U) sc = a.jobs[a.meta[slot].w >> 16].scene;
       float4 of = a.o[slot], df = a.d[slot];
-      V3 oo{of.x, of.y, of.z}, od{df.x, df.y, df.z};
+      const V3 o{of.x, of.y, of.z}, d{df.x, df.y, df.z};
+      // Panels and floor first: the nearest bounds the traversal (a hit of
+      // the piece at the same distance wins, as argent's order piece, panels,
+      // floor with strict comparisons keeps it), and the ray is at hand.
+      // After it, they reloaded the ray and the traversal went past the floor.
+      float t_pf = INFINITY;
+      pf = HIT_MISS;
+      for (int p = 0; p < sc->num_panels; ++p) {
+        const DevPanel& pn = sc->panels[p];
+        if (depth == 0 && !pn.camera_visible) continue;
+        float t;
+        if (panel_intersect(pn, o, d, t_pf, &t)) {
+          t_pf = t;
+          pf = HIT_PANEL | (uint32_t)p;
+        }
+      }
+      if (sc->floor_enabled) {
+        float t;
+        if (floor_intersect(sc, o, d, t_pf, &t)) {
+          t_pf = t;
+          pf = HIT_FLOOR;
+        }
+      }
+      V3 oo = o, od = d;
       if (U ? a.u_has_turn : sc->has_turn) {
         float ts = U ? a.u_to_obj_s : sc->to_obj_s, tc = U ? a.u_to_obj_c : sc->to_obj_c;
-        oo = rot_y_sc(oo, ts, tc);
-        od = rot_y_sc(od, ts, tc);
+        oo = rot_y_sc(o, ts, tc);
+        od = rot_y_sc(d, ts, tc);
       }
-      running = closest_begin(U ? a.upiece : sc->piece, s, oo, od, INFINITY);
+      running = closest_begin(U ? a.upiece : sc->piece, s, oo, od, INFINITY, t_pf);
       active = true;
     }
     if (__ballot_sync(0xffffffffu, active) == 0 && !more) break;
@@ -641,8 +664,8 @@ __global__ void __launch_bounds__(128, ARGENT_TRAV_BLOCKS) k_intersect(WaveArgs 
       if (leaves ? at_leaf : at_node) running = closest_visit(U ? a.upiece : sc->piece, s, stack, a.status);
     }
     // Lanes whose traversal is over wait until ARGENT_FIN_BATCH of them (or
-    // every active lane) can record their hits together: the panel and
-    // floor tests and the queue appends then run once for many lanes.
+    // every active lane) can record their hits together: the queue appends
+    // then run once for many lanes.
     bool waiting = active && !running;
     unsigned wm = __ballot_sync(0xffffffffu, waiting);
     unsigned rm = __ballot_sync(0xffffffffu, active && running);
@@ -651,32 +674,13 @@ __global__ void __launch_bounds__(128, ARGENT_TRAV_BLOCKS) k_intersect(WaveArgs 
     int cls = -1;
     if (fin) {
       count_visits(0, s.n_nodes, s.n_tris);
-      float4 of = a.o[slot], df = a.d[slot];
-      V3 o{of.x, of.y, of.z}, d{df.x, df.y, df.z};
-      float t_max = INFINITY;
-      float4 rec = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(HIT_MISS));
-      cls = CLS_TERMINAL;
+      float4 rec;
       if (s.best.prim != ARGENT_NO_HIT_U) {
-        t_max = s.best.t;
         rec = make_float4(s.best.t, s.best.u, s.best.v, __uint_as_float(s.best.prim));
         cls = sc->mat_class[__ldg(&(U ? a.upiece : sc->piece).tri_idx[s.best.prim].w)];
-      }
-      for (int p = 0; p < sc->num_panels; ++p) {
-        const DevPanel& pn = sc->panels[p];
-        if (depth == 0 && !pn.camera_visible) continue;
-        float t;
-        if (panel_intersect(pn, o, d, t_max, &t)) {
-          t_max = t;
-          rec = make_float4(t, 0.0f, 0.0f, __uint_as_float(HIT_PANEL | (uint32_t)p));
-          cls = CLS_TERMINAL;
-        }
-      }
-      if (sc->floor_enabled) {
-        float t;
-        if (floor_intersect(sc, o, d, t_max, &t)) {
-          rec = make_float4(t, 0.0f, 0.0f, __uint_as_float(HIT_FLOOR));
-          cls = sc->floor_class;
-        }
+      } else {
+        rec = make_float4(pf == HIT_MISS ? 0.0f : s.best.t, 0.0f, 0.0f, __uint_as_float(pf));
+        cls = pf == HIT_FLOOR ? sc->floor_class : CLS_TERMINAL;
       }
       a.hit[slot] = rec;
       active = false;
