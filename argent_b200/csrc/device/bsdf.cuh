@@ -212,7 +212,9 @@ __device__ __forceinline__ void bsdf_prepare(Bsdf& b, V3 wo) {
     b.wo_lam = ggx_lambda(b.ggx, wo);
   }
   if (KM_HAS(KM, B_CONDUCTOR) && b.kind == B_CONDUCTOR && !is_smooth(b.ggx) && wo.z > 0.0f) {
-    Spec f0 = fresnel_conductor(1.0f, b.eta, b.k);
+    Spec f0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) f0.v[i] = fresnel_conductor_normal(b.eta.v[i], b.k.v[i]);
     float e = ggx_e(b.ggx, wo.z);
     b.ms = spec(1.0f) + f0 * ((1.0f - e) / e);
     b.wo_lam = ggx_lambda(b.ggx, wo);

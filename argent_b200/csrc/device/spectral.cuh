@@ -206,6 +206,18 @@ __device__ __forceinline__ float fresnel_conductor1(float cos_theta_i, float eta
   float rs_im = (n2_im * d2_re - n2_re * d2_im) / dd2;
   return 0.5f * ((rp_re * rp_re + rp_im * rp_im) + (rs_re * rs_re + rs_im * rs_im));
 }
+// fresnel_conductor1 at normal incidence, bit for bit.  There sin^2 is 0, so
+// cos_t is (1, +-0) and e cos_t is e itself; r_perp's numerator is then
+// exactly minus r_parl's over the same denominator, and the mean of two equal
+// squares is either: |(e - 1) / (e + 1)|^2 as r_parl rounds it, in two divisions
+// instead of nine.
+__device__ __forceinline__ float fresnel_conductor_normal(float eta, float k) {
+  float n_re = eta - 1.0f, d_re = eta + 1.0f;
+  float dd = d_re * d_re + k * k;
+  float r_re = (n_re * d_re + k * k) / dd;
+  float r_im = (k * d_re - n_re * k) / dd;
+  return r_re * r_re + r_im * r_im;
+}
 __device__ __forceinline__ Spec fresnel_conductor(float c, const Spec& eta, const Spec& k) {
   Spec r;
 #pragma unroll
