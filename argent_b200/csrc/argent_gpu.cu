@@ -1247,7 +1247,10 @@ static int ensure_tables(ArgentCtx* ctx) {
       }
   ARGENT_CK(ctx, cudaMemcpyToSymbol(dev::d_sobol_bytes, bytes, sizeof(bytes)));
   ARGENT_CK(ctx, cudaMemcpyToSymbol(dev::d_energy_table, energy, sizeof(energy)));
-  ARGENT_CK(ctx, cudaMemcpyToSymbol(dev::d_cmf, ARGENT_CMF_1931_2DEG, sizeof(float) * 471 * 3));
+  std::vector<float4> cmf(471);
+  const float* c3 = ARGENT_CMF_1931_2DEG;
+  for (int i = 0; i < 471; ++i) cmf[i] = make_float4(c3[3 * i], c3[3 * i + 1], c3[3 * i + 2], 0.0f);
+  ARGENT_CK(ctx, cudaMemcpyToSymbol(dev::d_cmf, cmf.data(), cmf.size() * sizeof(float4)));
   ctx->tables_ready = true;
   return ARGENT_OK;
 }

@@ -307,11 +307,10 @@ __device__ __forceinline__ void xyz_bar(float lambda, float out[3]) {
   int i = (int)x;
   i = i > 469 ? 469 : i;
   float t = x - (float)i;
-  const float* a = d_cmf + 3 * i;
-  const float* b = a + 3;
-  out[0] = a[0] + (b[0] - a[0]) * t;
-  out[1] = a[1] + (b[1] - a[1]) * t;
-  out[2] = a[2] + (b[2] - a[2]) * t;
+  const float4 a = __ldg(d_cmf + i), b = __ldg(d_cmf + i + 1);
+  out[0] = a.x + (b.x - a.x) * t;
+  out[1] = a.y + (b.y - a.y) * t;
+  out[2] = a.z + (b.z - a.z) * t;
 }
 __device__ __forceinline__ void to_xyz(const Spec& l, const Wavelengths& wl, float xyz[3]) {
   xyz[0] = xyz[1] = xyz[2] = 0.0f;

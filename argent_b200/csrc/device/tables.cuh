@@ -14,8 +14,9 @@ __device__ uint32_t d_sobol_dirs[4][32];
 __device__ uint32_t d_sobol_bytes[4][4][256];
 // GGX single-scattering albedo E(mu, sqrt(alpha)), 32 x 32 (microfacet.rs:93-140).
 __device__ float d_energy_table[32 * 32];
-// CIE 1931 2-degree colour matching functions, 1 nm, 360..=830 (cie.rs:38-49).
-__device__ float d_cmf[471 * 3];
+// CIE 1931 2-degree colour matching functions (x, y, z, 0), 1 nm, 360..=830
+// (cie.rs:38-49): one 16-byte load per entry.
+__device__ float4 d_cmf[471];
 // Traversal instrumentation (off unless the host enables it): closest-hit
 // rays, nodes, triangles; any-hit rays, nodes, triangles.  The switch is in
 // constant memory: every node visit tests it.

@@ -1521,9 +1521,10 @@ __device__ __forceinline__ void ld_pair(const float4* p, bool aligned, bool two,
 // two at a time so that every 32-byte sector is fetched once and whole.  The
 // sums of a block's groups meet in shared memory, where one thread per pixel
 // and channel adds them to the film.  Bound by the instructions of the XYZ
-// projection (80 B per path at 3 times the copy rate's time): 7.7 ms per
-// 265 M paths of the signet still; one lane per sample with shuffles took
-// 8.9 ms.
+// projection and its table lookups (80 B per path at under twice the copy
+// rate's time): 6.0 ms per 265 M paths of the signet still, 7.6 with three
+// 4-byte loads per colour matching entry instead of one of 16, 8.9 with one
+// lane per sample and shuffles.
 __global__ void __launch_bounds__(256) k_film(WaveArgs a, WaveDesc w) {
   __shared__ float part[9][256];
   __shared__ double part64[3][256];
