@@ -1710,6 +1710,20 @@ static int run_jobs(ArgentCtx* ctx, const std::vector<dev::DevJob>& jobs, const 
   const int last_lane = (int)((start + waves.size() - 1) % nlanes);
   cudaStream_t join = joined ? ctx->stream : ctx->aux_stream;
 
+  // How far the kernels of a bounce run beside each other: 2 the shading
+  // classes and the shadow rays, 1 the shadow rays, 0 not at all (with timing
+  // on, too: every kernel then runs alone).  Few waves leave the device to the
+  // slowest ray of each kernel, so theirs fork; more waves overlap each other.
+  // A lane's streams share eight hardware queues with the other lanes', and
+  // waiting streams in one queue hold each other up: four waves of five
+  // streams ran the gems at 60.0 ms, of two at 52.4, one at 53.3.  Forked
+  // batches are launched directly: captured as a graph, their branches made
+  // its instantiation so slow that a new scene's first pass took 4.9 ms where
+  // the preview's repeated ones took 2.2, and 386 instead of 261 for the signet
+  // still; launched directly, 2.2 and 2.2 (and the signet still, which does not
+  // fork, 273 and 263).
+  const int forks = ctx->prof.on ? 0 : waves.size() <= 2 ? 2 : waves.size() <= 4 ? 1 : 0;
+
   // Issues the batch: fork from the context stream, each wave's kernels on
   // its lane, join.  Counts the kernels it launches.
   // The step of the issue that failed first, for the error text.
@@ -1771,9 +1785,9 @@ static int run_jobs(ArgentCtx* ctx, const std::vector<dev::DevJob>& jobs, const 
       // A small wave's time is the sum of its kernels' slowest rays and
       // paths, and a bounce is then two of them in a row instead of five or
       // six (preview of 1 M paths 2.84 -> 2.20 ms, ring still 1.68 -> 1.39,
-      // reel frame 18.4 -> 17.5, gems 57.4 -> 54.9; the signet still, whose
-      // eight lanes overlap anyway, unchanged).  With timing on, every kernel runs alone on the lane's stream.
-      const bool fork = !ctx->prof.on;
+      // reel frame 18.4 -> 17.5; the signet still, whose eight lanes overlap
+      // anyway, unchanged).  With timing on, every kernel runs alone on the lane's stream.
+      const bool fork = forks > 0, fork_classes = forks > 1;
       cudaStream_t* side = ctx->side_stream[lane];
       cudaEvent_t* sev = ctx->side_ev[lane];
       auto after = [&](cudaStream_t to, cudaEvent_t ev, cudaStream_t from) {  // `to` goes on after `from`
@@ -1817,7 +1831,7 @@ static int run_jobs(ArgentCtx* ctx, const std::vector<dev::DevJob>& jobs, const 
           for (int c = NUM_CLS - 1; c >= 0; --c) {
             if (!(classes & (1u << c))) continue;
             cudaStream_t sc = st;
-            if (fork && n > 0 && used_sides < ARGENT_SIDES - 1) {
+            if (fork_classes && n > 0 && used_sides < ARGENT_SIDES - 1) {
               sc = side[used_sides];
               if (used_sides == 0 && e == cudaSuccess) e = cudaEventRecord(sev[ARGENT_SIDES], st);
               if (e == cudaSuccess) e = cudaStreamWaitEvent(sc, sev[ARGENT_SIDES], 0);
@@ -1892,10 +1906,10 @@ static int run_jobs(ArgentCtx* ctx, const std::vector<dev::DevJob>& jobs, const 
 
   cudaError_t e = cudaSuccess;
   uint64_t kernels = 0;
-  // A joined batch without instrumentation is captured once as a CUDA graph
-  // and replayed while the same waves come again (a render repeated with new
+  // A joined batch without instrumentation whose bounces do not fork is
+  // captured once as a CUDA graph and replayed while the same waves come again (a render repeated with new
   // films, cameras or seeds changes only the job records).
-  const bool graphs = joined && !chain_first && !ctx->prof.on && !ctx->counting && ctx->graphs_on;
+  const bool graphs = joined && !chain_first && !ctx->prof.on && !ctx->counting && ctx->graphs_on && forks == 0;
   if (graphs) {
     std::vector<uint8_t> key;
     auto put = [&](const void* p, size_t n) {

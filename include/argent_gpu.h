@@ -668,9 +668,9 @@ int argent_ctx_set_profiling(ArgentCtx* ctx, int on);
 /* Summed device time (ms) and launch count per kernel class since the last
  * reset; synchronises the stream.  ms and launches hold ARGENT_KC_COUNT. */
 int argent_ctx_kernel_times(ArgentCtx* ctx, double* ms, uint64_t* launches);
-/* Renders that are not overlapped and not instrumented are captured as CUDA
- * graphs and replayed when the same waves come again (on by default); off
- * also frees the captured graphs. */
+/* Renders that are not overlapped and not instrumented and take more than
+ * four waves are captured as CUDA graphs and replayed when the same waves come
+ * again (on by default); off also frees the captured graphs. */
 int argent_ctx_set_graphs(ArgentCtx* ctx, int on);
 /* Ray sharing for batches (off by default).  argent's reel renders every
  * metal variant of a frame on its own (jobs.rs:595-713); variants that differ
