@@ -402,7 +402,8 @@ __global__ void __launch_bounds__(128) k_collapse(Collapse c, Bin bn, uint32_t n
     child_base = __shfl_sync(full, child_base, (int)g0);
     tri_base = __shfl_sync(full, tri_base, (int)g0);
     out_base = __shfl_sync(full, out_base, (int)g0);
-    uint32_t q[6] = {0, 0, 0, 0, 0, 0};  // this child's planes: lo x, y, z then hi x, y, z
+    // This child's planes: lo x, y, z then hi x, y, z (absent: inside out).
+    uint32_t q[6] = {255, 255, 255, 0, 0, 0};
     if (have) {
       for (int a = 0; a < 3; ++a) {
         q[a] = quant_lo(lo[a], klo[a], e[a]);

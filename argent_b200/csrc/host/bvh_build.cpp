@@ -317,6 +317,12 @@ struct Collapser {
     w.ex = e[0];
     w.ey = e[1];
     w.ez = e[2];
+    // Absent children: boxes inside out, which no ray enters.
+    for (size_t c = kids.size(); c < 8; ++c)
+      for (int a = 0; a < 3; ++a) {
+        w.qlo[a][c] = 255;
+        w.qhi[a][c] = 0;
+      }
     uint32_t n_interior = 0;
     for (uint32_t k : kids)
       if (!as_leaf(bn[k])) ++n_interior;
@@ -386,7 +392,7 @@ WideBvh build_wide_bvh(const float* positions, uint32_t nv, const uint32_t* tris
     out.hi[a] = nodes[root].box.hi[a];
   }
   out.nodes.reserve(nodes.size() / 4 + 1);
-  out.tris.reserve(nt);
+  out.tris.reserve((size_t)nt + 1);  // and the null record the upload adds
   out.nodes.resize(1);
   Collapser c{nodes, ref, positions, tris, out};
   out.depth = c.fill(0, root);
