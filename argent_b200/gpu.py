@@ -5,6 +5,7 @@ These mirror argent's own objects: `Piece` (scene.rs:10-38), `Scene`
 (render.rs:67-115), so callers and tests read like argent's.
 """
 
+import collections
 import ctypes
 import threading
 import weakref
@@ -29,7 +30,10 @@ class ResultPool:
     memory.  A block goes back to the pool once no array refers to it any more
     (any thread may drop the last one).  At most LIMIT bytes are page-locked in
     all; results beyond that, and those under SMALL bytes, are ordinary arrays.
-    At most IDLE bytes wait unused, the rest is freed."""
+    At most IDLE bytes wait unused: the sizes that came back longest ago are
+    freed first, so a program that moves to other sizes gets its own kept.
+    (Locking pages anew on each call costs more than the copy saves: three
+    334 x 1182 films 13-22 ms instead of 0.4 ms.)"""
 
     SMALL = 1 << 16
     LIMIT = 1 << 30
@@ -39,7 +43,7 @@ class ResultPool:
         # Reentrant: the garbage collector may finalise an array, and so
         # return its block, while this thread holds the lock.
         self._lock = threading.RLock()
-        self._free = {}  # block size -> addresses
+        self._free = collections.OrderedDict()  # block size -> addresses, last returned last
         self.total = 0  # bytes page-locked
         self.idle = 0  # of these, waiting
 
@@ -58,13 +62,10 @@ class ResultPool:
         if n < self.SMALL:
             return np.empty(shape, dtype)
         size = self._block(n)
-        ptr = None
         with self._lock:
-            if self._free.get(size):
-                ptr = self._free[size].pop()
-                self.idle -= size
-            else:
-                self._trim(size)
+            ptr = self._pop(size)
+            if ptr is None:
+                self._trim(lambda: self.total + size > self.LIMIT)
                 if self.total + size > self.LIMIT:
                     return np.empty(shape, dtype)
                 self.total += size
@@ -79,12 +80,20 @@ class ResultPool:
         weakref.finalize(buf, self._give, ptr, size).atexit = False
         return np.frombuffer(buf, dtype, count).reshape(shape)
 
-    def _trim(self, size):
-        """Frees waiting blocks of other sizes until `size` more bytes fit."""
-        for k in sorted(self._free):
-            while self._free[k] and self.total + size > self.LIMIT:
-                self._release(self._free[k].pop(), k)
-                self.idle -= k
+    def _pop(self, size):
+        """A waiting block of this size, or None."""
+        try:
+            ptr = self._free[size].pop()
+        except (KeyError, IndexError):
+            return None
+        self.idle -= size
+        return ptr
+
+    def _trim(self, over):
+        """Frees waiting blocks, the sizes used longest ago first, while over()."""
+        for k in tuple(self._free):
+            while over() and (ptr := self._pop(k)) is not None:
+                self._release(ptr, k)
 
     def _release(self, ptr, size):
         N.gpu().argent_pinned_free(ptr)
@@ -92,11 +101,10 @@ class ResultPool:
 
     def _give(self, ptr, size):
         with self._lock:
-            if self.idle + size > self.IDLE:
-                self._release(ptr, size)
-            else:
-                self._free.setdefault(size, []).append(ptr)
-                self.idle += size
+            self._free.setdefault(size, []).append(ptr)
+            self._free.move_to_end(size)
+            self.idle += size
+            self._trim(lambda: self.idle > self.IDLE)
 
 
 _results = ResultPool()

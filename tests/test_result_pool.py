@@ -69,6 +69,20 @@ def test_bounds_and_fallbacks(pool):
     assert pool.array((0, 4), np.float32).shape == (0, 4)
 
 
+def test_waiting_blocks_of_old_sizes_make_room(pool):
+    pool.IDLE = 3 << 20
+    held = [pool.array(1 << 20, np.uint8) for _ in range(3)]
+    del held
+    gc.collect()
+    assert pool.idle == pool.IDLE
+    a = pool.array(3 << 19, np.uint8)
+    del a
+    gc.collect()
+    assert pool.idle <= pool.IDLE and pool.total == pool.idle == sum(len(b) for b in pool.live.values())
+    pool.lib.fail = True  # nothing can be page-locked anew: the block was kept
+    assert not pool.array(3 << 19, np.uint8).flags.owndata
+
+
 def test_threads(pool):
     def work(k):
         for i in range(50):
