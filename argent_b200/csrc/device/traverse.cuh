@@ -5,15 +5,23 @@
 // Exactness.  The triangle test is argent's Moller-Trumbore in argent's
 // operation order (bvh.rs:391-410), rounded exactly like the f32 Rust code
 // (the library is compiled with --fmad=false).  The closest hit is the
-// minimum of (t, original triangle index) over all triangles that pass the
-// test, which does not depend on the tree; argent instead keeps the first of
-// equal-t hits in its own traversal order, and the parity tests bucket such
-// exact ties.  The tree only decides which triangles are tested, so box
-// culling must be conservative: child boxes are quantised outward (decoded
-// lo <= true lo, decoded hi >= true hi), and the slab interval is widened by
-// a bound on its own rounding error (node_ray), so a box whose exact
-// interval holds a hit distance is entered whenever argent's slab test
+// minimum of (t, original triangle index) over the triangles that are tested
+// and pass; argent instead keeps the first of equal-t hits in its own
+// traversal order, and the parity tests bucket such exact ties.  The boxes
+// decide which triangles are tested: child boxes are quantised outward
+// (decoded lo <= true lo, decoded hi >= true hi), and the slab interval is
+// widened by a bound on its own rounding error (node_ray), so a box whose
+// exact interval holds a hit distance is entered whenever argent's slab test
 // (bvh.rs:280-299), whose rounding is within that bound, would enter it.
+//
+// That covers every hit whose point lies in its triangle's box.  A triangle
+// seen edge-on can pass the test at a point outside its box, as its t, u and v
+// are then off by more than the interval is widened; whether such a hit is
+// found depends on the tree and on how the planes round (some 7 in 10^8 camera
+// rays of a still can change hit with the boxes, one in 10^9 did when the
+// planes were rounded on a coarser grid).  So the rounding of the planes is
+// part of the result: make_rayq, axis_q and child_q are not to be changed but
+// to forms of the same values (tests/test_box_arithmetic.py).
 #pragma once
 #include "dev_math.cuh"
 #include "tables.cuh"
@@ -156,6 +164,7 @@ struct NodeView {
 // share of what passes through L2 (path state streams through it once per
 // kernel), so nodes are kept in preference to the streaming data.
 __device__ __forceinline__ uint4 ld_node16(const uint4* ptr) {
+#ifdef __CUDA_ARCH__
   uint4 r;
   uint64_t pol;
   asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
@@ -163,6 +172,9 @@ __device__ __forceinline__ uint4 ld_node16(const uint4* ptr) {
       : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
       : "l"(ptr), "l"(pol));
   return r;
+#else
+  return *ptr;
+#endif
 }
 
 __device__ __forceinline__ NodeView load_node(const uint4* nodes, uint32_t idx) {
@@ -200,44 +212,35 @@ __device__ __forceinline__ uint32_t child_ref(const NodeView& n, int c) {
   return ARGENT_LEAF_BIT | (cnt1 << 27) | (n.tri_base + off);
 }
 
-// Byte c of the packed plane words (w0: children 0-3, w1: 4-7) as the exact
-// float 2^15 + byte, in one byte permute (integer-to-float conversions issue
-// on the narrow XU pipe): the byte lands on the mantissa bits of weight 1.
-// The slab test's biases absorb the 2^15 (AxisQ).
-#define ARGENT_PLANE_BIAS 32768.0f
+// Byte c of the packed plane words (w0: children 0-3, w1: 4-7) as an exact
+// float, without an integer-to-float conversion (those issue on the narrow
+// XU pipe): the byte is placed in the mantissa of 2^23, and 2^23 is
+// subtracted exactly.
 __device__ __forceinline__ float qf(uint32_t w0, uint32_t w1, int c) {
-  return __uint_as_float(__byte_perm(c < 4 ? w0 : w1, 0x47000000u, 0x7604u | ((uint32_t)(c & 3) << 4)));
+  return __fadd_rn(__uint_as_float(__byte_perm(c < 4 ? w0 : w1, 0x4B000000u, 0x7440u | (uint32_t)(c & 3))),
+                   -8388608.0f);
 }
 
 // A ray prepared for the node-space slab test: the inverse direction with
-// magnitudes capped (a zero component gives +-cap, so no 0 * inf arises),
-// and per axis whether the ray runs toward -axis.
+// magnitudes capped at 2^64 (a zero component gives +-2^64, so no 0 * inf
+// arises), and per axis whether the ray runs toward -axis.
 struct RayQ {
   V3 o;
   float ix, iy, iz;
   bool nx, ny, nz;
 };
 
-// The inverses come from the hardware's reciprocal estimate (1 ulp): the slab
-// interval's slack covers its error many times over, and hits do not depend
-// on the boxes beyond their being entered.
-__device__ __forceinline__ float capped_inv(float d, float cap) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-  return fminf(fmaxf(r, -cap), cap);
+__device__ __forceinline__ float capped_inv(float d) {
+  const float cap = 18446744073709551616.0f;  // 2^64
+  return fminf(fmaxf(__frcp_rn(d), -cap), cap);
 }
 
-// `root` is the word of the root node with its exponent bytes: pieces whose
-// boxes are so large that scale * cap * 2^15 could overflow (scale >= 2^33)
-// take a smaller cap.
-__device__ __forceinline__ RayQ make_rayq(V3 o, V3 d, uint32_t root) {
-  const bool big = (root & ((root << 1) | (root << 2)) & 0x00808080u) != 0;
-  const float cap = big ? 281474976710656.0f : 18446744073709551616.0f;  // 2^48, 2^64
+__device__ __forceinline__ RayQ make_rayq(V3 o, V3 d) {
   RayQ r;
   r.o = o;
-  r.ix = capped_inv(d.x, cap);
-  r.iy = capped_inv(d.y, cap);
-  r.iz = capped_inv(d.z, cap);
+  r.ix = capped_inv(d.x);
+  r.iy = capped_inv(d.y);
+  r.iz = capped_inv(d.z);
   r.nx = signbit(r.ix);
   r.ny = signbit(r.iy);
   r.nz = signbit(r.iz);
@@ -247,30 +250,39 @@ __device__ __forceinline__ RayQ make_rayq(V3 o, V3 d, uint32_t root) {
 // Three-operand minimum and maximum (one instruction on sm_100; a NaN operand
 // is dropped, as fminf and fmaxf drop it).
 __device__ __forceinline__ float min3(float a, float b, float c) {
+#ifdef __CUDA_ARCH__
   float r;
   asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
+#else
+  return fminf(fminf(a, b), c);
+#endif
 }
 __device__ __forceinline__ float max3(float a, float b, float c) {
+#ifdef __CUDA_ARCH__
   float r;
   asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
+#else
+  return fmaxf(fmaxf(a, b), c);
+#endif
 }
 
 // One axis of a node seen from a ray.  A plane q of the axis is at
 // t = (origin + q * scale - o) * inv = q * a + b, with a = scale * inv
-// (exact: scale is a power of two) and b = (origin - o) * inv.  It is
-// computed from the decoded v = 2^15 + q as fma(v, a, b'), b' = b - 2^15 a.
-// Against the exact value that is off by at most about
-// 2^-21 * |origin - o| * |inv| + 2^-9 * |a| (the roundings of b and b', the
-// inverse's ulp, the final rounding); the slack e = 2^-18 * |origin - o| *
-// |inv| + 2^-7 * |a| is over four times that, and is subtracted from the
-// near plane's bias and added to the far plane's (1/128 of a quantisation
-// step).  The near plane is the low one unless the ray runs toward -axis.
-// The traversals are bound by issue, the narrow integer pipe first, so the
-// decode is one permute, the bounds take three-operand min and max, and
-// children are counted from the sorted keys: the signet still's closest hit
-// went from 159.7 to 154.0 ms per frame, its shadow rays from 79.3 to 76.4.
+// (exact: scale is a power of two) and b = (origin - o) * inv.  Computed as
+// fma(q, a, b), t differs from the exact value by at most about
+// 3 * 2^-24 * (|origin - o| + 255 * scale) * |inv|; the slack e is 2^-18
+// times that magnitude (64 units of rounding), and is subtracted from the
+// near plane's bias and added to the far plane's.  The near plane is the
+// low one unless the ray runs toward -axis.
+//
+// The traversals are bound by issue.  Decoding a byte as 2^15 + q and carrying
+// the 2^15 in the biases saves the subtraction of each plane, but rounds them
+// on a coarser grid, which moved hits: signet still at 128 spp 129.0 ms so,
+// 132.0 with exact planes and inverses (the inverse by __frcp_rn, the same value
+// as the division, which took 132.7).  Planes in packed pairs (add and fma
+// f32x2) gave the same values in 134.4.
 struct AxisQ {
   float a, bn, bf;
   uint32_t n0, n1, f0, f1;
@@ -281,10 +293,10 @@ __device__ __forceinline__ AxisQ axis_q(float origin, float scale, float o, floa
   AxisQ q;
   float dd = __fsub_rn(origin, o);
   float b = __fmul_rn(dd, inv);
-  float e = __fmul_rn(__fmaf_rn(fabsf(dd), 3.814697265625e-06f, __fmul_rn(scale, 0.0078125f)), fabsf(inv));
+  float e = __fmul_rn(__fmul_rn(__fadd_rn(fabsf(dd), __fmul_rn(256.0f, scale)), fabsf(inv)), 3.814697265625e-06f);
   q.a = __fmul_rn(scale, inv);
-  q.bn = __fmaf_rn(-ARGENT_PLANE_BIAS, q.a, __fsub_rn(b, e));
-  q.bf = __fmaf_rn(-ARGENT_PLANE_BIAS, q.a, __fadd_rn(b, e));
+  q.bn = __fsub_rn(b, e);
+  q.bf = __fadd_rn(b, e);
   q.n0 = neg ? hi0 : lo0;
   q.n1 = neg ? hi1 : lo1;
   q.f0 = neg ? lo0 : hi0;
@@ -397,9 +409,11 @@ __device__ __forceinline__ void sort8(uint32_t k[8]) {
 // distance with its 3 low mantissa bits replaced by the child slot; the
 // truncated distance is what the stack keeps for pruning, which can only
 // keep more nodes than the exact value.
-// The visit order changes how much is pruned, never the result: a triangle
-// whose hit is the final best has box entry <= that distance <= the running
-// best at every point, so its box is always entered.
+// The visit order changes how much is pruned, not the result: a triangle
+// whose hit is the final best and lies in its box has box entry <= that
+// distance <= the running best at every point, so its box is always entered.
+// (A hit outside its box may be pruned by another within the distance between
+// the two; the order of visits is therefore the same in every form.)
 //
 // The traversal is resumable: closest_begin sets it up and each
 // closest_visit visits one node or one leaf, so a kernel can interleave the
@@ -418,8 +432,9 @@ struct ClosestTrav {
 
 // Returns false when the traversal is already over (empty piece, or a ray
 // that misses the piece's box); s.best is then a miss.  `limit` <= t_max is
-// the distance of something else the ray hits: a hit of the piece at most that
-// far is found, one beyond it need not be (s.best.t is then the limit).
+// the distance of something else the ray hits: boxes entered at most that far
+// are visited, so a hit of the piece up to there is found, and one beyond it
+// need not be (s.best.t is then the limit).
 __device__ __forceinline__ bool closest_begin(const DevPiece& pc, ClosestTrav& s, V3 o, V3 d, float t_max,
                                               float limit) {
   s.o = o;
@@ -433,7 +448,7 @@ __device__ __forceinline__ bool closest_begin(const DevPiece& pc, ClosestTrav& s
   s.n_tris = 0;
   if (pc.num_tris == 0) return false;
   const uint4 root = ld_node16(pc.nodes);
-  s.rq = make_rayq(o, d, root.w);
+  s.rq = make_rayq(o, d);
   if (!node_box_hit(root, s.rq, limit)) return false;
   s.have = true;
   return true;
@@ -544,7 +559,7 @@ struct AnyTrav {
 __device__ __forceinline__ bool piece_may_occlude(const DevPiece& pc, V3 o, V3 d, float t_max) {
   if (pc.num_tris == 0) return false;
   const uint4 root = ld_node16(pc.nodes);
-  return node_box_hit(root, make_rayq(o, d, root.w), t_max);
+  return node_box_hit(root, make_rayq(o, d), t_max);
 }
 
 // Returns ARGENT_ANY_RUNNING, or ARGENT_ANY_CLEAR when the ray misses the
@@ -560,7 +575,7 @@ __device__ __forceinline__ int any_begin(const DevPiece& pc, AnyTrav& s, ST& sta
   s.n_tris = 0;
   if (pc.num_tris == 0) return ARGENT_ANY_CLEAR;
   const uint4 root = ld_node16(pc.nodes);
-  s.rq = make_rayq(o, d, root.w);
+  s.rq = make_rayq(o, d);
   if (!node_box_hit(root, s.rq, t_max)) return ARGENT_ANY_CLEAR;
   stack.push(s.sp, 0u);
   return ARGENT_ANY_RUNNING;
@@ -623,9 +638,9 @@ __device__ __forceinline__ int any_visit(const DevPiece& pc, AnyTrav& s, ST& sta
 // chain of steps is several times shorter in time (a lone lane takes the
 // eight slab tests, the sort and the leaf's triangles one after the other).
 // All lanes of a warp call together; the lanes of a group pass the same ray.
-// The hits are those of a thread per ray: the closest hit is the
-// minimum of (t, triangle index) whatever the order of visits, and the boxes
-// are tested by the same arithmetic.
+// The hits are those of a thread per ray: the boxes are tested by the same
+// arithmetic and visited in the same order, and of a leaf's hits the minimum of
+// (t, triangle index) is kept.
 //
 // Rays are dealt to warps one by one first (coop_rays_per_warp), so with
 // fewer rays than warps the groups of a warp do not wait for each other.
@@ -669,7 +684,7 @@ __device__ __forceinline__ void coop_begin(const DevPiece& pc, CoopTrav& s, bool
   s.run = false;
   if (active && pc.num_tris != 0) {
     const uint4 root = ld_node16(pc.nodes);
-    s.rq = make_rayq(o, d, root.w);
+    s.rq = make_rayq(o, d);
     s.run = node_box_hit(root, s.rq, t_max);
   }
   s.have = s.run;

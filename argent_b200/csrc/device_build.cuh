@@ -8,9 +8,10 @@
 // builder does (open the interior child of largest area until 8 children;
 // subtrees of at most 4 triangles become leaves), level by level, writing
 // the same 80-byte node and 48-byte triangle layouts (host/bvh_build.h) with
-// the same conservative plane quantisation.  The traversal does not depend
-// on which builder made the tree: every closest hit is the minimum of
-// (t, triangle index) over the triangles whose Moller-Trumbore test passes.
+// the same conservative plane quantisation.  The traversal takes either
+// builder's tree: every closest hit is the minimum of (t, triangle index) over
+// the triangles that are tested and pass, which is the same for both but for
+// hits of edge-on triangles outside their own boxes (device/traverse.cuh).
 #pragma once
 #include <cuda_runtime.h>
 

@@ -3,7 +3,7 @@
 // Binary stage: binned SAH over all three axes (16 bins), leaves of at most
 // 4 triangles, built in parallel over subtrees.  Unlike argent's build
 // (bvh.rs:419-495, longest axis only), every axis is binned, which gives a
-// cheaper tree for the same triangles; closest hits do not depend on the tree.
+// cheaper tree for the same triangles.
 // Past depth 48 the build falls back to median splits so the tree depth, and
 // with it the device traversal stack, stays bounded.
 //
