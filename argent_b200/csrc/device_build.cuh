@@ -289,7 +289,10 @@ __global__ void __launch_bounds__(128) k_collapse(Collapse c, Bin bn, uint32_t n
     int nk = 0;
     auto take = [&](int32_t b) {
       kid = b;
-      area = leafish(bn, n, b) ? -1.0f : half_area(bn, b);
+      // A box that overflows (its piece is refused below) can have no number as
+      // its area, which must not enter the lanes' maximum: they would disagree.
+      const float a = leafish(bn, n, b) ? -1.0f : half_area(bn, b);
+      area = a >= 0.0f ? a : -1.0f;
     };
     if (on) {
       if (leafish(bn, n, item.y)) {
