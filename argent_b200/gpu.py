@@ -22,18 +22,17 @@ def _p(a, t=ctypes.c_void_p):
 
 
 class ResultPool:
-    """Arrays for results, in page-locked memory that is used again.
+    """Arrays in page-locked memory that is used again, for a program that
+    asks for them (its inputs, or results it reads through the C calls).
 
-    A result copied into fresh pageable memory pays for the driver's staging
-    copy and for the first touch of every page: a 1920 x 1080 film's three
-    images took 15 ms of a 300 ms render, and take 1.5 ms into page-locked
-    memory.  A block goes back to the pool once no array refers to it any more
-    (any thread may drop the last one).  At most LIMIT bytes are page-locked in
-    all; results beyond that, and those under SMALL bytes, are ordinary arrays.
-    At most IDLE bytes wait unused: the sizes that came back longest ago are
-    freed first, so a program that moves to other sizes gets its own kept.
-    (Locking pages anew on each call costs more than the copy saves: three
-    334 x 1182 films 13-22 ms instead of 0.4 ms.)"""
+    A block goes back to the pool once no array refers to it any more (any
+    thread may drop the last one), and the next array of its size is handed the
+    same memory: whoever starts an asynchronous copy out of such an array keeps
+    it until the copy is done.  At most LIMIT bytes are page-locked in all;
+    arrays beyond that, and those under SMALL bytes, are ordinary ones.  At
+    most IDLE bytes wait unused: the sizes that came back longest ago are freed
+    first, so a program that moves to other sizes gets its own kept.
+    (Locking and unlocking 25 MB takes 12 ms.)"""
 
     SMALL = 1 << 16
     LIMIT = 1 << 30
@@ -44,7 +43,7 @@ class ResultPool:
         # return its block, while this thread holds the lock.
         self._lock = threading.RLock()
         self._free = collections.OrderedDict()  # block size -> addresses, last returned last
-        self.total = 0  # bytes page-locked
+        self.total = 0  # bytes of all blocks
         self.idle = 0  # of these, waiting
 
     @staticmethod
@@ -70,15 +69,22 @@ class ResultPool:
                     return np.empty(shape, dtype)
                 self.total += size
         if ptr is None:
-            p = ctypes.c_void_p()
-            if N.gpu().argent_pinned_alloc(size, ctypes.byref(p)) != N.OK:
+            ptr = self._make(size)
+            if ptr is None:
                 with self._lock:
                     self.total -= size
                 return np.empty(shape, dtype)
-            ptr = p.value
         buf = (ctypes.c_char * size).from_address(ptr)
         weakref.finalize(buf, self._give, ptr, size).atexit = False
         return np.frombuffer(buf, dtype, count).reshape(shape)
+
+    def _make(self, size):
+        """The address of a new block, or None."""
+        p = ctypes.c_void_p()
+        return p.value if N.gpu().argent_pinned_alloc(size, ctypes.byref(p)) == N.OK else None
+
+    def _unmake(self, ptr):
+        N.gpu().argent_pinned_free(ptr)
 
     def _pop(self, size):
         """A waiting block of this size, or None."""
@@ -96,7 +102,7 @@ class ResultPool:
                 self._release(ptr, k)
 
     def _release(self, ptr, size):
-        N.gpu().argent_pinned_free(ptr)
+        self._unmake(ptr)
         self.total -= size
 
     def _give(self, ptr, size):
@@ -107,7 +113,34 @@ class ResultPool:
             self._trim(lambda: self.idle > self.IDLE)
 
 
-_results = ResultPool()
+class HostPool(ResultPool):
+    """The same in ordinary memory, for the results of the calls below.
+
+    Fresh arrays pay for the first touch of every page: a 1920 x 1080 film's
+    three images are read in 15.7 ms into new arrays and in 3.9 ms into blocks
+    used before.  Page-locked blocks would take 1.4 ms, but an asynchronous copy
+    out of a result (torch's non_blocking) would then still read it after the
+    array is dropped or written to, where one out of ordinary memory is staged
+    before it returns; and a program's first results would pay for the locking
+    (half a millisecond per MB)."""
+
+    def __init__(self):
+        super().__init__()
+        self._blocks = {}  # address -> the array whose memory it is
+
+    def _make(self, size):
+        try:
+            a = np.empty(size, np.uint8)
+        except MemoryError:
+            return None
+        self._blocks[a.ctypes.data] = a
+        return a.ctypes.data
+
+    def _unmake(self, ptr):
+        del self._blocks[ptr]
+
+
+_results = HostPool()
 
 
 class Context:

@@ -232,7 +232,7 @@ void* argent_ctx_stream(ArgentCtx* ctx);
 /* Page-locked host memory.  Results read into it (films, hits, images) come
  * straight from the device, without the driver's staging copy; it costs time
  * to make, so keep and reuse it.  Freed with argent_pinned_free, from any
- * thread, once no call writes to it. */
+ * thread, once no call writes to it and no asynchronous copy reads it. */
 int argent_pinned_alloc(size_t bytes, void** out);
 void argent_pinned_free(void* p);
 
