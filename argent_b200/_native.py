@@ -161,6 +161,7 @@ GPU_FUNCS = {
     "argent_ctx_destroy": (None, [ctypes.c_void_p]),
     "argent_last_error": (ctypes.c_char_p, [ctypes.c_void_p]),
     "argent_ctx_sync": (ctypes.c_int, [ctypes.c_void_p]),
+    "argent_ctx_trim": (ctypes.c_int, [ctypes.c_void_p]),
     "argent_ctx_stream": (ctypes.c_void_p, [ctypes.c_void_p]),
     "argent_ctx_kernel_launches": (ctypes.c_uint64, [ctypes.c_void_p]),
     "argent_piece_upload": (ctypes.c_int, [ctypes.c_void_p, c_float_p, ctypes.c_uint32, c_float_p, c_u32_p,

@@ -497,6 +497,14 @@ int argent_ctx_sync(ArgentCtx* ctx) {
   return ctx_check_status(ctx);
 }
 
+int argent_ctx_trim(ArgentCtx* ctx) {
+  if (!ctx) return set_error(nullptr, ARGENT_E_INVALID, "NULL argument");
+  ARGENT_CK(ctx, cudaSetDevice(ctx->device));
+  ARGENT_CK(ctx, cudaStreamSynchronize(ctx->stream));
+  ARGENT_CK(ctx, cudaMemPoolTrimTo(ctx->scratch, 0));
+  return ARGENT_OK;
+}
+
 int argent_pinned_alloc(size_t bytes, void** out) {
   if (!out || bytes == 0) return set_error(nullptr, ARGENT_E_INVALID, "argent_pinned_alloc: NULL argument or no bytes");
   *out = nullptr;

@@ -101,6 +101,11 @@ class ResultPool:
             while over() and (ptr := self._pop(k)) is not None:
                 self._release(ptr, k)
 
+    def trim(self):
+        """Frees the blocks that wait unused."""
+        with self._lock:
+            self._trim(lambda: True)
+
     def _release(self, ptr, size):
         self._unmake(ptr)
         self.total -= size
@@ -185,6 +190,12 @@ class Context:
 
     def sync(self):
         self.check(self.lib.argent_ctx_sync(self.h))
+
+    def trim(self):
+        """Gives back what waits to be used again: the context's device scratch
+        and the process's idle result memory."""
+        self.check(self.lib.argent_ctx_trim(self.h))
+        _results.trim()
 
     @property
     def kernel_launches(self):

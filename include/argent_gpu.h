@@ -227,6 +227,10 @@ void argent_ctx_destroy(ArgentCtx* ctx);
 const char* argent_last_error(const ArgentCtx* ctx);
 /* Block until the context's stream is idle. */
 int argent_ctx_sync(ArgentCtx* ctx);
+/* Gives the device scratch kept between calls (rays and hits, images, build
+ * temporaries; at most 1 GiB) back to the device, for other contexts, libraries
+ * or processes; the next calls take it anew.  Waits for the context stream. */
+int argent_ctx_trim(ArgentCtx* ctx);
 /* The context's cudaStream_t, as a void pointer. */
 void* argent_ctx_stream(ArgentCtx* ctx);
 /* Page-locked host memory.  Results read into it (films, hits, images) come

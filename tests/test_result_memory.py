@@ -60,3 +60,34 @@ def test_asynchronous_copies_of_dropped_results():
     for g, w in zip(got, want):
         assert np.array_equal(g.cpu().numpy().view(np.uint32), w.view(np.uint32))
     assert not torch.from_numpy(piece.trace_closest(sets[0])).is_pinned()
+
+
+def test_trim_frees_what_waits():
+    from argent_b200 import gpu as G
+
+    pool = type(G._results)()
+    held = [pool.array((n, 1 << 18), np.uint8) for n in (1, 2, 3)]
+    del held[:2]
+    gc.collect()
+    assert pool.idle > 0
+    pool.trim()
+    assert pool.idle == 0 and pool.total == held[0].nbytes and len(pool._blocks) == 1
+    held[0][:] = 1
+
+
+@pytest.mark.gpu
+def test_trim_gives_device_scratch_back():
+    import torch
+
+    from argent_b200.gpu import Context, denoise_atrous
+
+    ctx = Context(0)
+    small = np.ones((8, 8, 3), np.float32)
+    want = denoise_atrous(ctx, small)
+    ctx.trim()
+    free = torch.cuda.mem_get_info(0)[0]
+    denoise_atrous(ctx, np.ones((1500, 2000, 3), np.float32))
+    assert free - torch.cuda.mem_get_info(0)[0] > 100 << 20  # 28 floats a pixel stay
+    ctx.trim()
+    assert free - torch.cuda.mem_get_info(0)[0] < 8 << 20
+    assert np.array_equal(denoise_atrous(ctx, small), want)
