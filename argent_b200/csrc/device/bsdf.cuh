@@ -90,10 +90,12 @@ __device__ __forceinline__ void coated_eval_pdf(const Bsdf& b, V3 wo, V3 wi, Spe
 // to the caller) and *pdf = the visible-normal density of the half vector over
 // 4 wo.h.  With so = wo.z sqrt(1 + a^2 tan^2 wo) and si alike, G2 / (4 wo.z
 // wi.z) = 1 / (2 (wi.z so + wo.z si)) and G1(wo) / (4 wo.z) = 1 / (2 (wo.z +
-// so)), so one division serves both where the factors one by one take nine.
-// Light samples only: their values scale radiance and steer no path.  h.z and
-// the denominator of D, whose rounding a smooth surface amplifies, are
-// computed as everywhere else.
+// so)): two divisions where the factors one by one take nine.  (One division
+// for both, by x * y, left the pdf's largest error at 4.0e-7 where the factors'
+// is 3.6e-7; by two it is 3.4e-7, mean 5.7e-8 against 6.5e-8.  Signet still at
+// 128 spp 131.8 ms with one, 132.3 with two.)  Light samples only: their values
+// scale radiance and steer no path.  h.z and the denominator of D, whose
+// rounding a smooth surface amplifies, are computed as everywhere else.
 __device__ __forceinline__ void ggx_nee(Ggx g, float wo_lam, V3 wo, V3 wi, V3 h, float* spec_out, float* pdf) {
   const float a2 = g.alpha * g.alpha;
   const float c2 = h.z * h.z;
@@ -101,9 +103,9 @@ __device__ __forceinline__ void ggx_nee(Ggx g, float wo_lam, V3 wo, V3 wi, V3 h,
   const float so = wo.z * (1.0f + 2.0f * wo_lam);
   const float si = sqrtf(__fmaf_rn(a2, fmaxf(1.0f - wi.z * wi.z, 0.0f), wi.z * wi.z));
   const float x = __fmaf_rn(wi.z, so, wo.z * si), y = wo.z + so;
-  const float q = a2 / ((2.0f * ARGENT_PI_F) * (k * k) * (x * y));
-  *spec_out = q * y;
-  *pdf = q * x;
+  const float r = (2.0f * ARGENT_PI_F) * (k * k);
+  *spec_out = a2 / (r * x);
+  *pdf = a2 / (r * y);
 }
 
 // The coat's eval and pdf for a light sample (coated_eval_pdf but for

@@ -1502,14 +1502,16 @@ __global__ void k_count_bounces(const uint32_t* counters, int depths) {
 // Two neighbouring slots of a path array: one 32-byte load when the pair is
 // aligned to it (a whole sector per lane), else two of 16.
 __device__ __forceinline__ void ld_pair(const float4* p, bool aligned, bool two, float4* x, float4* y) {
+#ifdef __CUDA_ARCH__
   if (aligned && two) {
     asm("ld.global.L1::no_allocate.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
         : "=f"(x->x), "=f"(x->y), "=f"(x->z), "=f"(x->w), "=f"(y->x), "=f"(y->y), "=f"(y->z), "=f"(y->w)
         : "l"(p));
-  } else {
-    *x = __ldcs(p);
-    if (two) *y = __ldcs(p + 1);
+    return;
   }
+#endif
+  *x = __ldcs(p);
+  if (two) *y = __ldcs(p + 1);
 }
 
 // render.rs:96-111 + Film sums.  A pixel's samples are added in groups of

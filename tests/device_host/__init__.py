@@ -22,13 +22,14 @@ def compile_program(source, tmp_path, sanitize=False):
     with open(src, "w") as f:
         f.write(source)
     flags = ["-fsanitize=address,undefined", "-fno-sanitize-recover=undefined", "-g"] if sanitize else []
-    subprocess.run([cxx, "-std=c++20", "-O1", "-ffp-contract=off", "-pthread", *flags, "-I", HERE, "-I", ROOT, src,
-                    "-o", exe], check=True)
+    p = subprocess.run([cxx, "-std=c++20", "-O1", "-ffp-contract=off", "-pthread", *flags, "-I", HERE, "-I", ROOT, src,
+                        "-o", exe], capture_output=True, text=True)
+    assert p.returncode == 0, p.stderr[:3000]
     return exe
 
 
-def run(exe, data=b"", timeout=300):
+def run(exe, data=b"", args=(), timeout=300):
     """Runs a program on `data` (its standard input) and returns its output."""
-    p = subprocess.run([exe], input=data, stdout=subprocess.PIPE, stderr=subprocess.PIPE, timeout=timeout)
+    p = subprocess.run([exe, *args], input=data, stdout=subprocess.PIPE, stderr=subprocess.PIPE, timeout=timeout)
     assert p.returncode == 0, p.stderr.decode(errors="replace")[-3000:]
     return p.stdout
