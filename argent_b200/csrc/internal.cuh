@@ -222,7 +222,7 @@ struct ArgentCtx {
     uint64_t last_use;
   };
   std::vector<GraphEntry> graph_cache;
-  uint64_t graph_clock = 0;
+  uint64_t graph_clock = 0, graphs_captured = 0, graphs_launched = 0;
   bool graphs_on = true;
   // Batches trace the rays that renders have in common once
   // (argent_ctx_set_ray_sharing).

@@ -258,6 +258,12 @@ class Context:
         """Capture and replay repeated renders as CUDA graphs (default on)."""
         self.check(self.lib.argent_ctx_set_graphs(self.h, 1 if on else 0))
 
+    def graph_counts(self):
+        """(graphs captured, graph launches) since the context was created."""
+        a, b = ctypes.c_uint64(), ctypes.c_uint64()
+        self.check(self.lib.argent_ctx_graph_counts(self.h, ctypes.byref(a), ctypes.byref(b)))
+        return int(a.value), int(b.value)
+
     def set_ray_sharing(self, on):
         """Batches trace the rays their renders have in common once
         (argent_ctx_set_ray_sharing; default off)."""

@@ -676,6 +676,8 @@ int argent_ctx_kernel_times(ArgentCtx* ctx, double* ms, uint64_t* launches);
  * four waves are captured as CUDA graphs and replayed when the same waves come
  * again (on by default); off also frees the captured graphs. */
 int argent_ctx_set_graphs(ArgentCtx* ctx, int on);
+/* Graphs captured and graph launches since the context was created. */
+int argent_ctx_graph_counts(const ArgentCtx* ctx, uint64_t* captured, uint64_t* launched);
 /* Ray sharing for batches (off by default).  argent's reel renders every
  * metal variant of a frame on its own (jobs.rs:595-713); variants that differ
  * only in their materials -- the same piece, turntable angle, panels, floor,
