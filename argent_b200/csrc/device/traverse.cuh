@@ -516,7 +516,7 @@ __device__ __forceinline__ bool closest_visit(const DevPiece& pc, ClosestTrav& s
   }
   if (d_trav_counting) {
     int nh = 0;
-    for (int c = 0; c < 8; ++c) nh += k[c] != 0xFFFFFFFFu ? 1 : 0;
+    for (int c = 0; c < 8; ++c) nh += k[c] != 0xFFFFFFFFu && ((n.present >> c) & 1u) ? 1 : 0;
     atomicAdd(&d_trav_child_hits[nh], 1ull);
   }
   sort8(k);
@@ -747,6 +747,7 @@ __device__ __forceinline__ void coop_run(const DevPiece& pc, CoopTrav& s, ST& st
       const bool in = key != 0xFFFFFFFFu;
       // Far to near onto the stack; the nearest (rank 0) is entered next.
       const int nh = __popc((__ballot_sync(full, in) >> g0) & gmask);
+      if (d_trav_counting && s.run && !leaf && c == 0) atomicAdd(&d_trav_child_hits[(ANY ? 9 : 0) + nh], 1ull);
       if (s.run && s.sp + nh > ARGENT_STACK_SIZE) {  // refused at upload (see closest_visit)
         if (c == 0) atomicOr(status, ARGENT_STATUS_STACK_OVERFLOW);
         s.sp = 0;
@@ -784,7 +785,8 @@ __device__ __forceinline__ void coop_run(const DevPiece& pc, CoopTrav& s, ST& st
           key = ((unsigned long long)__float_as_uint(t) << 32) | prim;
         const unsigned hm = (__ballot_sync(full, key != ~0ull) >> g0) & gmask;
         if (ANY) {
-          if (hm) {
+          if (hm && s.run) {
+            s.n_tris -= cnt - (i0 + (uint32_t)__ffs((int)hm));  // counted up to the first hit, as any_visit does
             s.best.prim = 0;
             s.run = false;
           }
