@@ -233,11 +233,11 @@ __global__ void k_tri_records(float4* tris, const uint4* __restrict__ tri_idx, c
 struct CavityRays {
   const float4* pos;
   const float* normals;
-  uint32_t v0, n;  // first vertex of the launch, samples per vertex
+  uint32_t v0, k0, n;  // first vertex and sample of the launch, samples per vertex
   float distance, eps;
   uint32_t* counts;
   __device__ __forceinline__ bool ray(uint32_t j, V3* o, V3* dir, float* t_max) const {
-    const uint32_t v = v0 + j / n, k = j % n;
+    const uint32_t i = j + k0, v = v0 + i / n, k = i % n;
     float nx = normals[3 * (size_t)v], ny = normals[3 * (size_t)v + 1], nz = normals[3 * (size_t)v + 2];
     float rcp = __fdiv_rn(1.0f, __fsqrt_rn((nx * nx + ny * ny) + nz * nz));
     if (!(isfinite(rcp) && rcp > 0.0f)) return false;
@@ -265,7 +265,7 @@ struct CavityRays {
     return true;
   }
   __device__ __forceinline__ void done(uint32_t j, bool hit) const {
-    if (hit) atomicAdd(counts + v0 + j / n, 1u);
+    if (hit) atomicAdd(counts + v0 + (j + k0) / n, 1u);
   }
 };
 
@@ -1177,17 +1177,21 @@ int argent_piece_ambient_occlusion(ArgentCtx* ctx, ArgentPiece* piece, const flo
   ARGENT_CK(ctx, scratch_alloc(ctx, (void**)&d_ao, (size_t)nv * sizeof(float)));
   ARGENT_CK(ctx, cudaMemcpyAsync(d_n, normals, 3ull * nv * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
   ARGENT_CK(ctx, cudaMemsetAsync(d_cnt, 0, (size_t)nv * sizeof(uint32_t), ctx->stream));
-  // Launches of whole vertices, at most TRACE_CHUNK rays each.
+  // Launches of whole vertices, at most TRACE_CHUNK rays each, or of a part of
+  // one vertex's samples when it has more (the work counter has 32 bits and is
+  // raised past the end by every warp).
   const uint32_t step = (uint32_t)std::max<uint64_t>(1, TRACE_CHUNK / samples);
   uint64_t launches = 1;
-  for (uint64_t v = 0; v < nv; v += step, ++launches) {
-    const uint64_t m = (uint64_t)std::min<uint64_t>(step, nv - v) * samples;
-    CavityRays rays{piece->dev.pos, d_n, (uint32_t)v, samples, distance, eps, d_cnt};
-    ARGENT_CK(ctx, cudaMemsetAsync(ctx->d_status + TRACE_WORK, 0, sizeof(uint32_t), ctx->stream));
-    ProfScope ps(ctx, KC_TRACE);
-    k_cavity_ao<<<grid_for(ctx, (const void*)k_cavity_ao, 128, m), 128, 0, ctx->stream>>>(
-        piece->dev, rays, (uint32_t)m, ctx->d_status + TRACE_WORK, ctx->d_status);
-  }
+  for (uint64_t v = 0; v < nv; v += step)
+    for (uint64_t k = 0; k < samples; k += TRACE_CHUNK, ++launches) {
+      const uint64_t m =
+          samples > TRACE_CHUNK ? std::min(TRACE_CHUNK, samples - k) : std::min<uint64_t>(step, nv - v) * samples;
+      CavityRays rays{piece->dev.pos, d_n, (uint32_t)v, (uint32_t)k, samples, distance, eps, d_cnt};
+      ARGENT_CK(ctx, cudaMemsetAsync(ctx->d_status + TRACE_WORK, 0, sizeof(uint32_t), ctx->stream));
+      ProfScope ps(ctx, KC_TRACE);
+      k_cavity_ao<<<grid_for(ctx, (const void*)k_cavity_ao, 128, m), 128, 0, ctx->stream>>>(
+          piece->dev, rays, (uint32_t)m, ctx->d_status + TRACE_WORK, ctx->d_status);
+    }
   int g2 = (int)std::min<uint64_t>((nv + 255) / 256, (uint64_t)ctx->num_sms * 8);
   k_cavity_ao_finish<<<std::max(g2, 1), 256, 0, ctx->stream>>>(d_cnt, nv, samples, d_ao);
   ctx->launches += launches;
