@@ -578,7 +578,6 @@ int argent_piece_upload(ArgentCtx* ctx, const float* positions, uint32_t nv, con
   };
   void *dn = nullptr, *dt = nullptr, *dp = nullptr, *dnr = nullptr, *di = nullptr, *dc = nullptr;
   cudaError_t e = up(bvh.nodes.data(), bvh.nodes.size() * sizeof(argent::WideNode), &dn);
-  if (nt) bvh.tris.push_back(argent::TriRecord{});  // the null record behind the last (closest_visit)
   if (e == cudaSuccess) e = up(bvh.tris.data(), bvh.tris.size() * sizeof(argent::TriRecord), &dt);
   if (e == cudaSuccess) e = up(pos4.data(), pos4.size() * sizeof(float4), &dp);
   if (e == cudaSuccess && normals) e = up(nrm4.data(), nrm4.size() * sizeof(float4), &dnr);
@@ -776,7 +775,7 @@ int argent_piece_upload_device_bvh(ArgentCtx* ctx, const float* positions, uint3
   };
   const size_t o_pos = place((size_t)nv * sizeof(float4)), o_nrm = place(normals ? (size_t)nv * sizeof(float4) : 0),
                o_idx = place((size_t)nt * sizeof(uint4)), o_cav = place(cavity ? (size_t)nv * sizeof(float) : 0),
-               o_tri = place(((size_t)nt + 1) * sizeof(argent::TriRecord));
+               o_tri = place((size_t)nt * sizeof(argent::TriRecord));
   uint8_t* base = nullptr;
   cudaError_t e = device_alloc(ctx, (void**)&base, bytes);
   if (e != cudaSuccess)
@@ -808,8 +807,6 @@ int argent_piece_upload_device_bvh(ArgentCtx* ctx, const float* positions, uint3
     if (rm) up(rm, tri_material, (size_t)nt * sizeof(uint16_t));
     if (cavity) up(base + o_cav, cavity, (size_t)nv * sizeof(float));
     if (e == cudaSuccess) e = cudaMemsetAsync(info, 0, 2 * sizeof(uint32_t), st);
-    if (e == cudaSuccess)  // the null record behind the last
-      e = cudaMemsetAsync(base + o_tri + (size_t)nt * sizeof(argent::TriRecord), 0, sizeof(argent::TriRecord), st);
     if (e == cudaSuccess) {
       db::k_piece_pack<<<(uint32_t)ctx->num_sms * 8, 256, 0, st>>>(rp, rn, rt, rm, nv, nt, pos4, nrm4, tidx, info);
       ++ctx->launches;

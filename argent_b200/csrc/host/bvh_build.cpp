@@ -317,7 +317,8 @@ struct Collapser {
     w.ex = e[0];
     w.ey = e[1];
     w.ez = e[2];
-    // Absent children: boxes inside out, which no ray enters.
+    // Absent children: boxes inside out, which only far rays enter
+    // (closest_visit).
     for (size_t c = kids.size(); c < 8; ++c)
       for (int a = 0; a < 3; ++a) {
         w.qlo[a][c] = 255;
@@ -392,7 +393,7 @@ WideBvh build_wide_bvh(const float* positions, uint32_t nv, const uint32_t* tris
     out.hi[a] = nodes[root].box.hi[a];
   }
   out.nodes.reserve(nodes.size() / 4 + 1);
-  out.tris.reserve((size_t)nt + 1);  // and the null record the upload adds
+  out.tris.reserve(nt);
   out.nodes.resize(1);
   Collapser c{nodes, ref, positions, tris, out};
   out.depth = c.fill(0, root);

@@ -125,9 +125,9 @@ def _exact_mesh(n):
     return pos, np.concatenate([np.stack([a, b, c], -1), np.stack([a, c, d], -1)]).astype(np.uint32)
 
 
-def _edge_on(pos, tris, n, rng):
+def _edge_on(pos, tris, n, rng, far=9):
     """Rays through points of triangles' edges, nearly in the triangles'
-    planes: products, sums, quotients and square roots only (exactly rounded),
+    planes, from up to 2^far away: products, sums, quotients and square roots only (exactly rounded),
     powers of two by ldexp."""
     p = pos[tris[rng.integers(len(tris), size=n)]].astype(np.float64)
     e = p[:, 1] - p[:, 0]
@@ -139,10 +139,13 @@ def _edge_on(pos, tris, n, rng):
     d = d + nn * np.ldexp(rng.integers(-4096, 4096, (n, 1)) / 4096.0, -rng.integers(2, 24, (n, 1)))
     d = d / np.sqrt(d[:, :1] ** 2 + d[:, 1:2] ** 2 + d[:, 2:] ** 2)
     rays = np.zeros((n, 8), f)
-    rays[:, 0:3] = x - d * np.ldexp(1.0 + rng.integers(0, 4096, (n, 1)) / 4096.0, rng.integers(-2, 9, (n, 1)))
+    rays[:, 0:3] = x - d * np.ldexp(1.0 + rng.integers(0, 4096, (n, 1)) / 4096.0, rng.integers(-2, far, (n, 1)))
     rays[:, 3] = np.inf
     rays[:, 4:7] = d
     return rays
+
+
+FAR_HITS = {False: ("82fd223b06530502", "b3775b69ddcb8179"), True: ("0fc6ef50916f092d", "3f3445fdc5cd532f")}
 
 
 @pytest.mark.gpu
@@ -165,3 +168,26 @@ def test_hits_of_edge_on_rays_are_fixed():
         assert np.array_equal(piece.trace_closest(few).view(np.uint32), hits[:8192].view(np.uint32))
         assert np.array_equal(piece.trace_anyhit(few), occ[:8192])
     assert (closest.hexdigest()[:16], occluded.hexdigest()[:16]) == ("01f832b78b3112a0", "2e1877e372215214")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("device_bvh", [False, True])
+def test_hits_of_far_rays_are_fixed(device_bvh):
+    """Rays from up to 2^26 away, where a box is smaller than the interval's
+    widening (more of its node's boxes are entered, absent children's inside-out
+    ones too): recorded hits of both builders' trees, and the same from the form
+    for few rays."""
+    from argent_b200 import mesh as M
+    from argent_b200.gpu import Context, Piece
+
+    pos, tris = _exact_mesh(192)
+    piece = Piece(Context(0), M.Mesh(pos, tris, np.zeros_like(pos), np.zeros(len(tris), np.uint16)),
+                  device_bvh=device_bvh)
+    rays = _edge_on(pos, tris, 1 << 18, np.random.default_rng(12), far=26)
+    hits, occ = piece.trace_closest(rays), piece.trace_anyhit(rays)
+    for k in range(0, 1 << 16, 8192):
+        few = np.ascontiguousarray(rays[k:k + 8192])
+        assert np.array_equal(piece.trace_closest(few).view(np.uint32), hits[k:k + 8192].view(np.uint32))
+        assert np.array_equal(piece.trace_anyhit(few), occ[k:k + 8192])
+    got = tuple(hashlib.sha256(a.tobytes()).hexdigest()[:16] for a in (hits, occ))
+    assert got == FAR_HITS[device_bvh]
