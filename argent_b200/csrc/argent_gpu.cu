@@ -75,7 +75,7 @@ __device__ __forceinline__ void trace_closest_queue(const DevPiece& pc, uint32_t
       V3 o, d;
       float t_max;
       src.ray(j, &o, &d, &t_max);
-      running = closest_begin(pc, s, o, d, t_max, t_max);
+      running = closest_begin(pc, s, o, d, t_max);
       active = true;
     }
     if (__ballot_sync(0xffffffffu, active) == 0 && !more) break;

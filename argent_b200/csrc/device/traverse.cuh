@@ -431,16 +431,12 @@ struct ClosestTrav {
 };
 
 // Returns false when the traversal is already over (empty piece, or a ray
-// that misses the piece's box); s.best is then a miss.  `limit` <= t_max is
-// the distance of something else the ray hits: boxes entered at most that far
-// are visited, so a hit of the piece up to there is found, and one beyond it
-// need not be (s.best.t is then the limit).
-__device__ __forceinline__ bool closest_begin(const DevPiece& pc, ClosestTrav& s, V3 o, V3 d, float t_max,
-                                              float limit) {
+// that misses the piece's box); s.best is then a miss.
+__device__ __forceinline__ bool closest_begin(const DevPiece& pc, ClosestTrav& s, V3 o, V3 d, float t_max) {
   s.o = o;
   s.d = d;
   s.t_max = t_max;
-  s.best = TraceHit{limit, 0.0f, 0.0f, ARGENT_NO_HIT_U};
+  s.best = TraceHit{t_max, 0.0f, 0.0f, ARGENT_NO_HIT_U};
   s.ref = 0u;
   s.sp = 0;
   s.have = false;
@@ -449,7 +445,7 @@ __device__ __forceinline__ bool closest_begin(const DevPiece& pc, ClosestTrav& s
   if (pc.num_tris == 0) return false;
   const uint4 root = ld_node16(pc.nodes);
   s.rq = make_rayq(o, d);
-  if (!node_box_hit(root, s.rq, limit)) return false;
+  if (!node_box_hit(root, s.rq, t_max)) return false;
   s.have = true;
   return true;
 }

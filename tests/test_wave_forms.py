@@ -119,3 +119,31 @@ def test_graphs_of_map_and_gradient_waves():
             for got, ref in zip(render(b), w):
                 assert np.array_equal(got, ref)
             assert ctx.graph_counts() == ((k + 1, k + 1) if repeat == 0 else (2, k + 3))
+
+
+@pytest.mark.parametrize("away", [1.0, 1e3, 1e5])
+def test_camera_rays_of_a_far_camera(away):
+    """A small render's camera rays take eight lanes each, in a wave with a
+    larger render a lane each: the same hits, so the same film, also from so far
+    that hits and boxes are off by more than the panels and the floor are apart
+    (the camera moved back with its picture kept)."""
+    from argent_b200 import mesh as M
+    from argent_b200.gpu import Context, Film, Piece, Scene, render_batch, render_pass
+
+    m = M.ring()
+    ctx = Context(0)
+    piece = Piece(ctx, m)
+    cam, turn = W.shot(piece, W.hull(m), "hero", 100.0, 0.0, 1.0)
+    scene = Scene(ctx, piece, W._studio_scene(m, [W.metal("sterling", 0.07, 0.8)], "white", turn + 13.0))
+    dist = -float(np.dot(cam.pos, cam.forward))
+    for i in range(3):
+        cam.pos[i] -= cam.forward[i] * dist * (away - 1.0)
+    cam.half_w /= away
+    cam.half_h /= away
+    ps = W.settings(3)
+    for seed in range(24):  # 7744 camera rays: four per resident warp at most
+        alone, among, other = Film(ctx, 44, 44), Film(ctx, 44, 44), Film(ctx, 256, 256)
+        render_pass(ctx, scene, cam, alone, ps, 4, seed)
+        render_batch(ctx, [(scene, cam, among, ps, 4, seed), (scene, cam, other, ps, 4, seed)])
+        for a, b in zip([alone.xyz(), *alone.read()], [among.xyz(), *among.read()]):
+            assert a.any() and np.array_equal(a.view(np.uint32), b.view(np.uint32))
