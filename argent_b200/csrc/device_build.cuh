@@ -57,11 +57,11 @@ __global__ void __launch_bounds__(256) k_piece_pack(const float* __restrict__ po
   const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
   uint32_t bad = 0, top = 0;
   if (t0 < 6) info[2 + t0] = t0 < 3 ? 0xffffffffu : 0u;
-  for (uint32_t i = t0; i < nv; i += stride) {
-    const float x = pos[3 * (size_t)i], y = pos[3 * (size_t)i + 1], z = pos[3 * (size_t)i + 2];
+  for (uint64_t i = t0; i < nv; i += stride) {  // nv may be near 2^32, where a 32-bit i would wrap
+    const float x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
     if (!(isfinite(x) && isfinite(y) && isfinite(z))) bad |= DB_BAD_POSITION;
     pos4[i] = make_float4(x, y, z, 0.0f);
-    if (nrm) nrm4[i] = make_float4(nrm[3 * (size_t)i], nrm[3 * (size_t)i + 1], nrm[3 * (size_t)i + 2], 0.0f);
+    if (nrm) nrm4[i] = make_float4(nrm[3 * i], nrm[3 * i + 1], nrm[3 * i + 2], 0.0f);
   }
   for (uint32_t i = t0; i < nt; i += stride) {
     const uint32_t a = tri[3 * (size_t)i], b = tri[3 * (size_t)i + 1], c = tri[3 * (size_t)i + 2];
