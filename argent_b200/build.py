@@ -64,7 +64,7 @@ def _host_cxx():
 
 
 def build_gpu(force=False, verbose=False, out=None, defines=()):
-    """The CUDA library; `out` and `defines` (e.g. ["ARGENT_SHORT_STACK=8"])
+    """The CUDA library; `out` and `defines` (e.g. ["ARGENT_REFILL=24"])
     build a variant with other build-time constants at another path, which
     ARGENT_GPU_LIB then selects."""
     out = out or GPU_SO

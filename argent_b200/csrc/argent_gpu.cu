@@ -59,7 +59,7 @@ int set_error(const ArgentCtx* ctx, int code, const std::string& msg) {
 // whichever are more.  With a thread per ray a warp ran until its slowest ray
 // ended: a million rays from round and off a 2.1M-triangle piece took 955 us,
 // now 790-840 (ncu, cold), the patina mask's 6 M hemisphere rays on 250k
-// triangles 2100, now 1193.  `work` is zero at the start.
+// triangles 2100, now 1258.  `work` is zero at the start.
 template <class SRC>
 __device__ __forceinline__ void trace_closest_queue(const DevPiece& pc, uint32_t count, uint32_t* work, SRC src,
                                                     uint32_t* status) {

@@ -494,11 +494,6 @@ __device__ __forceinline__ uint32_t lane_refill(bool idle, bool* first, bool* mo
   return j < count ? j : ~0u;
 }
 
-// scene.rs:169-218: closest hit of every active path (piece BVH in object
-// space, then panels, then floor), then the path is queued for the shading
-// kernel of its hit's material class.  Persistent lanes step their BVH
-// traversals one node or leaf at a time and take a new path as soon as
-// theirs is done.
 // Eight lanes per ray, every ray of the queue at once (coop_trace): a queue
 // of up to 4 rays per resident warp leaves the device mostly idle, and its
 // time is that of its slowest ray.
@@ -595,6 +590,11 @@ __device__ __forceinline__ void intersect_few(const WaveArgs& a, int depth, uint
     warp_append(cls == k, slot, a.counters + CNT_CLS(depth, k), a.qc + (size_t)k * a.cap, a.cap, a.status);
 }
 
+// scene.rs:169-218: closest hit of every active path (panels, floor, and the
+// piece BVH in object space), then the path is queued for the shading
+// kernel of its hit's material class.  Persistent lanes step their BVH
+// traversals one node or leaf at a time and take a new path as soon as
+// theirs is done.
 template <bool U>
 __global__ void __launch_bounds__(128, ARGENT_TRAV_BLOCKS) k_intersect(WaveArgs a, int depth) {
   // With ray sharing, the rays that take their leader's hit are left out
