@@ -328,10 +328,20 @@ int grid_for(const ArgentCtx* ctx, const void* kernel, int block, uint64_t n) {
   return (int)std::max<uint64_t>(g, 1);
 }
 
-// Rays of one launch at most, and the status buffer's word that counts the
-// batches they are taken in.
+// Rays of one launch at most, the status buffer's word that counts the batches
+// they are taken in, and its words for launches that are being captured: a
+// graph may run beside the context's calls and other graphs, so each captured
+// launch has a word of its own (used again after that many captured launches).
 static constexpr uint64_t TRACE_CHUNK = 1ull << 30;
-static constexpr int TRACE_WORK = 2;
+static constexpr int TRACE_WORK = 2, TRACE_WORK_CAPTURED = 4;
+static constexpr uint32_t TRACE_CAPTURES = 1u << 16;
+
+static uint32_t* trace_work(ArgentCtx* ctx) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(ctx->stream, &st) != cudaSuccess || st == cudaStreamCaptureStatusNone)
+    return ctx->d_status + TRACE_WORK;
+  return ctx->d_status + TRACE_WORK_CAPTURED + ctx->captured_traces++ % TRACE_CAPTURES;
+}
 
 // Blocks of 128 threads for the eight-lanes-per-ray form of a trace of `n`
 // rays (every ray at once, one per warp while warps are free), or 0 when the
@@ -424,7 +434,7 @@ int argent_ctx_create(int device, const ArgentLimits* limits, ArgentCtx** out) {
   for (int l = 0; l < ctx->lanes && r == cudaSuccess; ++l)
     r = cudaEventCreateWithFlags(&ctx->film_ev[l], cudaEventDisableTiming);
   if (r == cudaSuccess) r = cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, device);
-  if (r == cudaSuccess) r = cudaMalloc(&ctx->d_status, sizeof(uint32_t) * 4);
+  if (r == cudaSuccess) r = cudaMalloc(&ctx->d_status, sizeof(uint32_t) * (TRACE_WORK_CAPTURED + TRACE_CAPTURES));
   if (r == cudaSuccess) r = cudaMemset(ctx->d_status, 0, sizeof(uint32_t) * 4);
   if (r == cudaSuccess) r = cudaMallocHost((void**)&ctx->h_status, 4096);
   if (r == cudaSuccess) {
@@ -871,10 +881,11 @@ static void launch_trace_closest(ArgentCtx* ctx, ArgentPiece* piece, const Argen
   }
   for (uint64_t at = 0; at < n; at += TRACE_CHUNK) {
     const uint32_t m = (uint32_t)std::min<uint64_t>(TRACE_CHUNK, n - at);
-    cudaMemsetAsync(ctx->d_status + TRACE_WORK, 0, sizeof(uint32_t), ctx->stream);
+    uint32_t* work = trace_work(ctx);
+    cudaMemsetAsync(work, 0, sizeof(uint32_t), ctx->stream);
     ProfScope ps(ctx, KC_TRACE);
     k_trace_closest<<<grid_for(ctx, (const void*)k_trace_closest, 128, m), 128, 0, ctx->stream>>>(
-        piece->dev, d_rays + at, m, d_hits + at, ctx->d_status + TRACE_WORK, ctx->d_status);
+        piece->dev, d_rays + at, m, d_hits + at, work, ctx->d_status);
   }
 }
 
@@ -900,10 +911,11 @@ int argent_trace_anyhit_device(ArgentCtx* ctx, ArgentPiece* piece, const ArgentR
   } else {
     for (uint64_t at = 0; at < n; at += TRACE_CHUNK) {
       const uint32_t m = (uint32_t)std::min<uint64_t>(TRACE_CHUNK, n - at);
-      ARGENT_CK(ctx, cudaMemsetAsync(ctx->d_status + TRACE_WORK, 0, sizeof(uint32_t), ctx->stream));
+      uint32_t* work = trace_work(ctx);
+      ARGENT_CK(ctx, cudaMemsetAsync(work, 0, sizeof(uint32_t), ctx->stream));
       ProfScope ps(ctx, KC_TRACE);
       k_trace_any<<<grid_for(ctx, (const void*)k_trace_any, 128, m), 128, 0, ctx->stream>>>(
-          piece->dev, d_rays + at, m, d_occ + at, ctx->d_status + TRACE_WORK, ctx->d_status);
+          piece->dev, d_rays + at, m, d_occ + at, work, ctx->d_status);
     }
   }
   ctx->launches++;

@@ -250,6 +250,7 @@ struct ArgentCtx {
   std::string err;
   uint64_t launches = 0;
   uint32_t* d_status = nullptr;
+  uint32_t captured_traces = 0;
   uint32_t* h_status = nullptr;  // page-locked words for small reads: the status, a build's counters
   // Stream-ordered scratch of single calls (rays and hits, images, build
   // temporaries): up to ARGENT_SCRATCH_KEEP bytes stay with the context between

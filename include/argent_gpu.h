@@ -350,7 +350,8 @@ int argent_trace_anyhit(ArgentCtx* ctx, ArgentPiece* piece, const ArgentRay* ray
  */
 int argent_trace_closest_noalloc(ArgentCtx* ctx, ArgentPiece* piece, const ArgentRay* rays, uint64_t n,
                                  ArgentHit* hits);
-/* Device-pointer variants (asynchronous on the context stream). */
+/* Device-pointer variants (asynchronous on the context stream; they may be
+ * captured into a graph, which may then run on any stream). */
 int argent_trace_closest_device(ArgentCtx* ctx, ArgentPiece* piece, const ArgentRay* d_rays, uint64_t n,
                                 ArgentHit* d_hits);
 int argent_trace_anyhit_device(ArgentCtx* ctx, ArgentPiece* piece, const ArgentRay* d_rays, uint64_t n,
